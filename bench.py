@@ -98,12 +98,12 @@ def measured_peak():
 
 # stage kernel launched by each launch shape (dgsem_autotune / --variant)
 VARIANT_KERNELS = {
-    0: "stage_kernel", 1: "stage_kernel", 2: "stage_kernel",
+    0: "stage_line_kernel", 1: "stage_line_kernel", 2: "stage_line_kernel",
     3: "stage_node_kernel", 4: "stage_node_kernel", 5: "stage_pipe_kernel",
     6: "stage_node2_kernel",
 }
 KERNEL_DESCRIPTIONS = {
-    "stage_kernel": "stage_kernel (line-parallel fused RHS + SSPRK3 stage)",
+    "stage_line_kernel": "stage_line_kernel (line sweeps, fused RHS + SSPRK3 stage)",
     "stage_node_kernel": "stage_node_kernel (node-parallel fused RHS + SSPRK3 stage)",
     "stage_pipe_kernel": "stage_pipe_kernel (persistent node-parallel, TMA tile streaming)",
     "stage_node2_kernel": "stage_node2_kernel (node-parallel, two nodes per thread)",
@@ -126,7 +126,7 @@ def profile_value(workload: str, kernel: str, key: str):
     return None
 
 
-def profile_traffic(workload: str, kernel: str = "stage_kernel"):
+def profile_traffic(workload: str, kernel: str = "stage_line_kernel"):
     return profile_value(workload, kernel, "traffic_bytes_per_launch")
 
 
@@ -609,7 +609,7 @@ def run_device_arm(args):
     mean_stage_s = sum(step_ms) / (3 * args.steps) * 1e-3
     achieved = dofs * bpd / mean_stage_s / 1e9
     peak, peak_kind = measured_peak()
-    kernel = VARIANT_KERNELS.get(variant, "stage_kernel")
+    kernel = VARIANT_KERNELS.get(variant, "stage_line_kernel")
     traffic = profile_traffic(name, kernel)
     # FP64 bound: FP64 operations per launch (ncu op counters of the committed
     # summary, per DOF) over the same average launch time, against the FP64

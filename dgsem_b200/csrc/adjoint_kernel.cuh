@@ -3,7 +3,7 @@
 //   R(u) = -1/J [ split-form volume (Chandrashekar) + LLF surface + lifting
 //                 (+ Navier-Stokes BR1 viscous terms) ]
 // i.e. the transpose of the linearisation of exactly the arithmetic of the
-// forward kernels (stage_kernel.cuh, br1_kernel.cuh); the forward operators
+// forward kernels (stage_line_kernel.cuh, br1_kernel.cuh); the forward operators
 // restate structured_solver.hpp:466-480, volume_flux.hpp:221-294,
 // surface_flux.hpp:45-127, surface_integral.hpp:35-80, jacobian.hpp:76-101,
 // parabolic_gradient.hpp:480-818 and parabolic_viscous.hpp:343-592.

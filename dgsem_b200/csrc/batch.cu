@@ -347,6 +347,9 @@ dgsem_status dgsem_batch_create(const dgsem_mesh_desc* meshes, int n_meshes,
   b->offsets.assign(n_meshes + 1, 0);
   std::vector<MetricTablesHost> mts(n_meshes);
   std::map<int, BasisTables> bases;
+  // every table starts on a 32-byte boundary (the line sweeps read metric rows
+  // and -1/J as vectors)
+  auto padded = [](size_t count) { return (count + 3) / 4 * 4; };
   size_t table_total = 0;
   for (int m = 0; m < n_meshes; ++m) {
     const dgsem_mesh_desc& d = meshes[m];
@@ -367,8 +370,8 @@ dgsem_status dgsem_batch_create(const dgsem_mesh_desc* meshes, int n_meshes,
     b->offsets[m + 1] = b->offsets[m] + ne * nodes * (nd + 2);
     by_n[n].push_back(m);
     for (int a = 0; a < nd; ++a) {
-      table_total += mts[m].coord[a].size() + mts[m].jdiag[a].size();
-      for (int c = 0; c < nd; ++c) table_total += mts[m].ja[a][c].size();
+      table_total += padded(mts[m].coord[a].size()) + padded(mts[m].jdiag[a].size());
+      for (int c = 0; c < nd; ++c) table_total += padded(mts[m].ja[a][c].size());
     }
   }
   double* tables = balloc<double>(b, table_total);
@@ -390,7 +393,7 @@ dgsem_status dgsem_batch_create(const dgsem_mesh_desc* meshes, int n_meshes,
   auto place = [&](const std::vector<double>& v) -> const double* {
     const double* dptr = tables + off;
     std::memcpy(host.data() + off, v.data(), v.size() * sizeof(double));
-    off += v.size();
+    off += padded(v.size());
     return dptr;
   };
   for (int m = 0; m < n_meshes; ++m)
@@ -454,7 +457,7 @@ dgsem_status dgsem_batch_create(const dgsem_mesh_desc* meshes, int n_meshes,
     int64_t nel_total = 0, nodes_total = 0;
     for (int m = 0; m < n_meshes; ++m) {
       nel_total += b->nelem[m];
-      nodes_total += b->nelem[m] * b->nodes[m];
+      nodes_total += (int64_t)padded((size_t)(b->nelem[m] * b->nodes[m]));
     }
     int* info = balloc<int>(b, (size_t)nel_total * 12);
     double* mij = info ? balloc<double>(b, (size_t)nodes_total) : nullptr;
@@ -479,7 +482,7 @@ dgsem_status dgsem_batch_create(const dgsem_mesh_desc* meshes, int n_meshes,
         b->minfo[m] = info + io;
         b->mmij[m] = mij + mo;
         io += b->nelem[m] * 12;
-        mo += b->nelem[m] * b->nodes[m];
+        mo += (int64_t)padded((size_t)(b->nelem[m] * b->nodes[m]));
       }
   }
   if (e == cudaSuccess) e = build_persistent(b);

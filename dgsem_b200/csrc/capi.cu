@@ -1,6 +1,6 @@
 // C ABI implementation: context lifetime, descriptor validation, device
 // tables, and the small auxiliary kernels (indicator, initial conditions,
-// layout conversion).  The fused stage kernel lives in stage_kernel.cuh.
+// layout conversion).  The fused stage kernels live in stage_*_kernel.cuh.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -340,9 +340,11 @@ dgsem_status dgsem_ctx_create(const dgsem_mesh_desc* mesh,
     delete ctx;
     return DGSEM_ERR_INVALID_ARG;
   }
-  // one device block for all tables
+  // one device block for all tables, each on a 32-byte boundary (the line
+  // sweeps read metric rows as vectors)
   size_t total = 0;
-  auto add = [&](const std::vector<double>& v) { total += v.size(); };
+  auto padded = [](size_t count) { return (count + 3) / 4 * 4; };
+  auto add = [&](const std::vector<double>& v) { total += padded(v.size()); };
   for (int a = 0; a < nd; ++a) {
     add(mt.coord[a]);
     add(mt.jdiag[a]);
@@ -362,7 +364,7 @@ dgsem_status dgsem_ctx_create(const dgsem_mesh_desc* mesh,
   auto place = [&](const std::vector<double>& v) -> const double* {
     const double* dptr = ctx->table_block + off;
     std::memcpy(host.data() + off, v.data(), v.size() * sizeof(double));
-    off += v.size();
+    off += padded(v.size());
     return dptr;
   };
   std::memset(&c.tab, 0, sizeof(c.tab));

@@ -15,6 +15,7 @@
 
 #include "br1_kernel.cuh"
 #include "stage_kernel.cuh"
+#include "stage_line_kernel.cuh"
 #include "stage_node2_kernel.cuh"
 #include "stage_node_kernel.cuh"
 #include "stage_pipe_kernel.cuh"
@@ -47,7 +48,7 @@ struct EngineConfig {
   int skip_tile_copy;
 };
 
-// Launch-shape variants: 0-2 line-parallel (stage_kernel.cuh), 3-4
+// Launch-shape variants: 0-2 line sweeps (stage_line_kernel.cuh), 3-4
 // node-parallel (stage_node_kernel.cuh), 5 persistent node-parallel with TMA
 // tile streaming (stage_pipe_kernel.cuh; single-mesh launches; split form
 // without shock capturing or viscous terms, an even number of doubles per
@@ -141,20 +142,13 @@ inline StageArgs<N> stage_args_common(const EngineConfig& cfg, double a, double 
   return args;
 }
 
-// Launch geometry per (DIM, N, variant): one thread per element line.
-//   variant 0: ~128 (2D) / ~96 (3D) threads per block, no register cap
-//   variant 1: same block, register cap for one more resident block per SM
-//   variant 2: twice the elements per block, no register cap
-template <int DIM, int N, int V>
-struct LaunchShape {
-  static constexpr int NLINE = DIM * ipow(N, DIM - 1);
-  static constexpr int TARGET = DIM == 2 ? 128 : 96;
-  static constexpr int EPB0 = (TARGET / NLINE) > 0 ? (TARGET / NLINE) : 1;
-  static constexpr int EPB = V == 2 ? 2 * EPB0 : EPB0;
-  static constexpr int NT = ((EPB * NLINE + 31) / 32) * 32;
-  // variant 1 caps registers at 65536 / (MINB * NT) (about 100 per thread);
-  // MINB = 0: no cap
-  static constexpr int MINB = V == 1 ? (65536 / (NT * 100) > 1 ? 65536 / (NT * 100) : 2) : 0;
+// Line-sweep variants 0-2 (stage_line_kernel): warps per block and resident
+// blocks per SM requested from the register allocator.
+template <int N, int V>
+struct LineLaunch {
+  static constexpr int WPB = V == 2 ? 4 : 2;
+  static constexpr int MINB = V == 0 ? 6 : V == 1 ? 8 : N > 4 ? 2 : 3;
+  static constexpr int NT = 32 * WPB;
 };
 
 // Fraction of the lanes of its warps that a block of `threads` threads uses.
@@ -211,39 +205,31 @@ class Engine final : public EngineBase {
  public:
   static constexpr int GRAD_EPB = (128 / ipow(N, DIM)) > 0 ? (128 / ipow(N, DIM)) : 1;
   static constexpr bool kBatch = !NS && !HG;
-  // the line-parallel shapes 0-2 carry shock capturing or the viscous terms
-  // in 2D only (not both); otherwise the node-parallel shapes run (0-2 then
-  // run shape 3)
-  static constexpr bool kLine = !(DIM == 3 && (HG || NS)) && !(HG && NS);
+  // the line-sweep shapes 0-2 have no viscous terms: with Navier-Stokes they
+  // run shape 3
+  static constexpr bool kLine = !NS;
 
-  template <int V>
-  using Sh = StageShape<DIM, N, VF, SF, HG, LaunchShape<DIM, N, V>::EPB, NS>;
-
-  template <int V>
-  static auto kernel() {
-    using L = LaunchShape<DIM, N, V>;
-    if constexpr (L::MINB == 0)
-      return stage_kernel<DIM, N, VF, SF, HG, L::EPB, L::NT, NS, false>;
-    else
-      return stage_kernel_capped<DIM, N, VF, SF, HG, L::EPB, L::NT, NS, false, L::MINB>;
+  template <int V, bool B>
+  static auto line_kernel() {
+    return stage_line_kernel<DIM, N, VF, SF, HG, B, LineLaunch<N, V>::WPB, LineLaunch<N, V>::MINB>;
   }
   template <int V>
-  static auto batch_kernel() {
-    using L = LaunchShape<DIM, N, V>;
-    if constexpr (L::MINB == 0)
-      return stage_kernel<DIM, N, VF, SF, HG, L::EPB, L::NT, NS, true>;
-    else
-      return stage_kernel_capped<DIM, N, VF, SF, HG, L::EPB, L::NT, NS, true, L::MINB>;
+  static constexpr size_t line_smem() {
+    return LineShape<DIM, N, VF>::smem_bytes(LineLaunch<N, V>::WPB);
+  }
+  template <int V>
+  static constexpr int line_epb() {
+    return LineGeo<DIM, N>::EPW * LineLaunch<N, V>::WPB;
   }
 
   template <int V>
   static void set_attributes() {
     if constexpr (kLine)
-      cudaFuncSetAttribute(kernel<V>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)Sh<V>::smem_bytes);
+      cudaFuncSetAttribute(line_kernel<V, false>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)line_smem<V>());
     if constexpr (kBatch)
-      cudaFuncSetAttribute(batch_kernel<V>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)Sh<V>::smem_bytes);
+      cudaFuncSetAttribute(line_kernel<V, true>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)line_smem<V>());
   }
 
   // node-parallel shapes: split form with shock capturing or with the
@@ -354,7 +340,11 @@ class Engine final : public EngineBase {
 
   StageArgs<N> common_args(const EngineConfig& cfg, double a, double b, double t,
                            const double* t_dev, double* alpha_out) const {
-    return stage_args_common<N>(cfg, a, b, t, t_dev, alpha_out);
+    StageArgs<N> args = stage_args_common<N>(cfg, a, b, t, t_dev, alpha_out);
+    for (int i = 0; i < N; ++i)
+      for (int j = 0; j < N; ++j)
+        args.basis.Dvol[i][j] = LineScale<VF>::value * args.basis.Dsplit[i][j];
+    return args;
   }
 
   template <int V>
@@ -362,10 +352,10 @@ class Engine final : public EngineBase {
     if constexpr (!kLine) {
       launch_node<true>(args, nelem, s);
     } else {
-      using L = LaunchShape<DIM, N, V>;
-      const int64_t blocks = (nelem + L::EPB - 1) / L::EPB;
+      const int64_t blocks = (nelem + line_epb<V>() - 1) / line_epb<V>();
       last_grid_ = blocks;
-      launch_stage_kernel(kernel<V>(), (unsigned)blocks, L::NT, Sh<V>::smem_bytes, s, args);
+      launch_stage_kernel(line_kernel<V, false>(), (unsigned)blocks, LineLaunch<N, V>::NT,
+                          line_smem<V>(), s, args);
     }
   }
 
@@ -422,8 +412,8 @@ class Engine final : public EngineBase {
   template <int V>
   void launch_batch(const StageArgs<N>& args, int ntiles, cudaStream_t s) const {
     if constexpr (kBatch) {
-      using L = LaunchShape<DIM, N, V>;
-      launch_stage_kernel(batch_kernel<V>(), (unsigned)ntiles, L::NT, Sh<V>::smem_bytes, s, args);
+      launch_stage_kernel(line_kernel<V, true>(), (unsigned)ntiles, LineLaunch<N, V>::NT,
+                          line_smem<V>(), s, args);
     }
   }
 
@@ -465,17 +455,17 @@ class Engine final : public EngineBase {
     if constexpr (kNode2)
       if (variant_ == 6) return Node2Launch<N>::EPB;
     if (variant_ >= 3 || !kLine) return NL::EPB;
-    return variant_ == 2 ? LaunchShape<DIM, N, 2>::EPB : LaunchShape<DIM, N, 0>::EPB;
+    return variant_ == 2 ? line_epb<2>() : line_epb<0>();
   }
   int threads_per_block() const override {
     if (variant_ >= 3 || !kLine) return NL::NT;
-    return variant_ == 2 ? LaunchShape<DIM, N, 2>::NT : LaunchShape<DIM, N, 0>::NT;
+    return variant_ == 2 ? LineLaunch<N, 2>::NT : LineLaunch<N, 0>::NT;
   }
   size_t smem_bytes() const override {
     if constexpr (kNode2)
       if (variant_ == 6) return Node2Shape<N, VF>::smem_bytes;
     if (variant_ >= 3 || !kLine) return NSh::smem_bytes;
-    return variant_ == 2 ? Sh<2>::smem_bytes : Sh<0>::smem_bytes;
+    return variant_ == 2 ? line_smem<2>() : line_smem<0>();
   }
   void set_variant(int v) override { variant_ = (v >= 0 && v < num_variants()) ? v : 0; }
   int variant() const override { return variant_; }

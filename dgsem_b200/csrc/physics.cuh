@@ -31,6 +31,43 @@ struct NodeState {
   double inv_rho;
 };
 
+// Branch-free reciprocal, quotient and square root of normal numbers: the
+// hardware's approximations (rcp.approx.ftz.f64, rsqrt.approx.ftz.f64, about
+// 20 bits) with one step of the third-order Newton-Schulz / Householder
+// iteration, 1/a = r (1 + e + e^2 + O(e^3)) with e = 1 - a r, and
+// sqrt(x) = g (1 + e/2 + 3 e^2/8 + O(e^3)) with g = x r, e = 1 - g r.  Within
+// one unit in the last place for arguments whose reciprocal is a normal
+// number (checked by the GPU tests); zero, infinite and subnormal arguments
+// give a NaN (reciprocal, quotient), root gives 0 below 1e-290.  The compiler's division and
+// sqrt carry a branch for those arguments, which ends a scheduling block at
+// every use.
+__device__ __forceinline__ double recip(double a) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(a));
+  const double e = __fma_rn(-a, r, 1.0);
+  return __fma_rn(r, __fma_rn(e, e, e), r);
+}
+
+// One Newton step: relative error about 1e-12.
+__device__ __forceinline__ double recip_approx(double a) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(a));
+  return __fma_rn(r, __fma_rn(-a, r, 1.0), r);
+}
+
+__device__ __forceinline__ double quotient(double a, double b) {
+  const double r = recip(b), q = __dmul_rn(a, r);
+  return __fma_rn(__fma_rn(-q, b, a), r, q);
+}
+
+__device__ __forceinline__ double root(double x) {
+  double r;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double g = __dmul_rn(x, r), e = __fma_rn(-g, r, 1.0);
+  const double s = __fma_rn(__dmul_rn(g, e), __fma_rn(0.375, e, 0.5), g);
+  return x < 1.0e-290 && x >= 0.0 ? 0.0 : s;
+}
+
 // Reciprocals of two nonzero quantities with one division, 1/(a b) times the
 // other factor.  The callers pass quantities of one pair of states (sums of
 // densities, pressures, rho p products or rho / p ratios; face normal

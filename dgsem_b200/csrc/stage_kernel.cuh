@@ -1,18 +1,12 @@
-// Fused DGSEM stage kernel for sm_100a: one launch computes, per element,
+// Shared parts of the fused DGSEM stage kernels for sm_100a: one launch
+// computes, per element,
 //   RHS(u_in) = -1/J [ sum_dir V_dir(u_in) + surface lift ]
 // and writes either du or the SSPRK3 stage value a*u_n + b*u_in + c*du.
-//
-// Per block: EPB elements, NT threads.  Phases (shared-memory staged):
-//   0  coalesced load of the block's contiguous u_in tile  [EPB][NV][ND]
-//   1  per-node primitives (v, p, beta, kin) and, with shock capturing, the
-//      Hennemann-Gassner alpha of each element
-//   2  (a) every face node of the element's 2*DIM faces: interface or
-//          boundary flux f*, the neighbour's trace read from L2;
-//      (b) every line of the element (DIM * n^(DIM-1) of them): symmetric
-//          split-form pair loop (each two-point flux evaluated once, both
-//          endpoints accumulated in registers) plus, for troubled elements,
-//          the FV subcell fluxes along the line and the alpha blend
-//   3  sum of directions + lifting, times -1/J, SSPRK3 combination, store.
+// Here: launch arguments, element and node indices, the Hennemann-Gassner
+// indicator, the fused diagnostics, boundary states and the interface flux of
+// the node-parallel kernels.  The kernels: stage_line_kernel.cuh (line
+// sweeps), stage_node_kernel.cuh, stage_node2_kernel.cuh, stage_pipe_kernel.cuh
+// (one or two nodes per thread).
 // Reference path replaced (one Kokkos kernel per item, :line):
 //   deep_copy(du, 0)                         solver/structured_solver.hpp:469
 //   HGIndicator2D                            subcell_limiting/indicator.hpp:337-418
@@ -37,6 +31,7 @@ __host__ __device__ constexpr int ipow(int b, int e) { return e == 0 ? 1 : b * i
 template <int N>
 struct BasisConst {
   double Dsplit[N][N];
+  double Dvol[N][N];  // Dsplit / 4 (Kennedy-Gruber) or / 2: line_pair_flux
   double Dhat[N][N];
   double Vinv[N][N];
   double inv_w[N];
@@ -334,8 +329,8 @@ __device__ __forceinline__ double hg_alpha_from_energies(double total, double c1
 
 // Sequential energy sums over m2[j*N + i] in the reference's order
 // (total over all modes, clip1 over j,i < N-1, clip2 over j,i < N-2).
-template <int N>
-__device__ __forceinline__ void hg_energy_sums(const double* m2, double* total, double* c1,
+template <int N, class Modes>
+__device__ __forceinline__ void hg_energy_sums(const Modes& m2, double* total, double* c1,
                                                double* c2) {
   double t = 0.0, a = 0.0, b = 0.0;
 #pragma unroll
@@ -359,8 +354,8 @@ __device__ __forceinline__ void hg_energy_sums(const double* m2, double* total, 
 // coverage (indicator.hpp:494-544): clip2 over i, j, k < N-2; clip1 adds the
 // index-(N-2) layers; total adds the layer k = N-1 and the rows j = N-1 of
 // k < N-1.
-template <int N>
-__device__ __forceinline__ void hg_energy_sums_3d(const double* m2, double* total, double* c1,
+template <int N, class Modes>
+__device__ __forceinline__ void hg_energy_sums_3d(const Modes& m2, double* total, double* c1,
                                                   double* c2) {
   auto at = [&](int k, int j, int i) { return m2[(k * N + j) * N + i]; };
   double b = 0.0;
@@ -479,13 +474,11 @@ __device__ double hg_alpha_2d(const double* us_el, int ND, const BasisConst<N>& 
 }
 
 // ---------------------------------------------------------------------------
-// The fused stage kernel
+// Shared by the stage kernels
 // ---------------------------------------------------------------------------
-// Shared-memory node arrays of the line-parallel kernel are padded by one
-// slot per N nodes (pnode = node + node / N) so that the per-line strided
-// accesses of the volume phase fall on distinct banks.  The node-parallel
-// kernels, whose warps read 32 consecutive nodes shifted along one line,
-// use the unpadded layout (PAD = false).
+// Node position in a shared-memory plane, optionally padded by one slot per N
+// nodes.  The node-parallel kernels, whose warps read 32 consecutive nodes
+// shifted along one line, use the unpadded layout (PAD = false).
 template <int N, bool PAD = true>
 __device__ __forceinline__ constexpr int padn(int node) {
   return PAD ? node + node / N : node;
@@ -541,41 +534,6 @@ __device__ __forceinline__ void load_element_tile(const double* src, double* us,
   t.issue(src, ne, tid);
   t.store(src, us, ne, tid);
 }
-
-// Per-node shared-memory slots: the velocity, the flux-specific scalars and
-// -1/J.  Chandrashekar needs (p, beta, kin), Ranocha (p), Kennedy-Gruber
-// (p, e); p is always present because the surface fluxes use it.
-template <int DIM, int VF>
-struct NodeSlots {
-  static constexpr int P = DIM;
-  static constexpr int BETA = DIM + 1;  // beta (Chandrashekar) or e (Kennedy-Gruber)
-  static constexpr int KIN = DIM + 2;   // Chandrashekar only
-  static constexpr int NQ_FLUX = VF == VF_CHANDRASHEKAR ? DIM + 3
-                                 : VF == VF_KENNEDY_GRUBER ? DIM + 2 : DIM + 1;
-  static constexpr int MIJ = NQ_FLUX;   // -1/J
-  static constexpr int NQ = NQ_FLUX + 1;
-};
-
-template <int DIM, int N, int VF, int SF, bool HG, int EPB, bool NS = false>
-struct StageShape {
-  static constexpr int NV = DIM + 2;
-  static constexpr int ND = ipow(N, DIM);
-  static constexpr int NDP = ND + ND / N;  // padded node count
-  static constexpr int NF = ipow(N, DIM - 1);
-  static constexpr int NFACE = 2 * DIM;
-  static constexpr int NLINE = DIM * NF;
-  static constexpr int NQ = NodeSlots<DIM, VF>::NQ;
-  static constexpr int SM_U = EPB * NV * NDP;
-  static constexpr int SM_P = EPB * NQ * NDP;
-  static constexpr int SM_V = EPB * DIM * NV * NDP;
-  static constexpr int SM_A = EPB;
-  static constexpr int SM_W = NS ? EPB * DIM * NV * NDP : 0;  // -F_v [el][dim][var][node]
-  // per element int info: ijk[3], eidx_other[3], neighbour[6] (-1 = boundary)
-  static constexpr int NI = 12;
-  static constexpr int SM_VINV = HG ? N * N : 0;
-  static constexpr size_t smem_bytes =
-      sizeof(double) * (SM_U + SM_P + SM_V + SM_A + SM_W + SM_VINV) + sizeof(int) * EPB * NI;
-};
 
 // Navier-Stokes pieces used by the stage kernel (defined in br1_kernel.cuh).
 __device__ __forceinline__ void ns_gradient_variables(const double* u, double gamma,
@@ -729,429 +687,6 @@ __device__ __forceinline__ void element_face_flux_state(
         f[v] += wv_el[(0 * NV + v) * NDP + opn] * nrm[0] + wv_el[(1 * NV + v) * NDP + opn] * nrm[1];
     }
   }
-}
-
-// element_face_flux_state with the own state taken from the line-parallel
-// kernel's shared memory (conserved tile + NodeSlots primitives).
-template <int DIM, int N, int VF, int SF, bool NS, int NDP>
-__device__ __forceinline__ void element_face_flux(
-    const StageArgs<N>& p, const MeshView& M, const double* us_el, const double* pr_el, const double* wv_el,
-    const int* I, int dir, int side, int line, double gamma, double t_stage, int c0, int c1,
-    int c2, double* f) {
-  constexpr int NV = DIM + 2;
-  using Q = NodeSlots<DIM, VF>;
-  const int opn = padn<N>(line_node<DIM, N>(dir, line, side ? N - 1 : 0));
-  FaceState<DIM> so;
-#pragma unroll
-  for (int q = 0; q < NV; ++q) so.u[q] = us_el[q * NDP + opn];
-#pragma unroll
-  for (int d = 0; d < DIM; ++d) so.v[d] = pr_el[d * NDP + opn];
-  so.p = pr_el[Q::P * NDP + opn];
-  so.a2 = gamma * so.p / so.u[0];
-  element_face_flux_state<DIM, N, VF, SF, NS, NDP>(p, M, so, us_el, wv_el, I, dir, side, line,
-                                                   gamma, t_stage, c0, c1, c2, f);
-}
-
-// One line of direction DIR of element el: symmetric split-form pair loop
-// (each two-point flux evaluated once, both end nodes accumulated in
-// registers), viscous / FV terms, and the surface fluxes of the two faces the
-// line ends on, lifted into its end nodes.  DIR is a compile-time constant:
-// tasks are ordered direction-major so a warp never mixes directions.
-template <int DIR, int DIM, int N, int VF, int SF, bool HG, bool NS, int NDP, int NQ, int NI>
-__device__ __forceinline__ void process_line(const StageArgs<N>& p, const MeshView& M,
-                                             const double* us,
-                                             const double* pr, double* dv,
-                                             const double* alpha_s, const double* wv,
-                                             const int* info, int el, int line, double gamma,
-                                             double t_stage, int c0, int c1, int c2) {
-  constexpr int NV = DIM + 2, ND = ipow(N, DIM);
-  using Q = NodeSlots<DIM, VF>;
-  constexpr int dir = DIR;
-  const int* I = info + el * NI;
-  const double* U = us + el * NV * NDP;
-  const double* P = pr + el * NQ * NDP;
-  double acc[N][NV];
-#pragma unroll
-  for (int m = 0; m < N; ++m)
-#pragma unroll
-    for (int q = 0; q < NV; ++q) acc[m][q] = 0.0;
-  double ja[N][DIM];
-#pragma unroll
-  for (int c = 0; c < DIM; ++c) {
-    const double* tab = M.tab.ja[dir][c] + (int64_t)I[3 + c] * ND;
-#pragma unroll
-    for (int m = 0; m < N; ++m) ja[m][c] = __ldg(tab + line_node<DIM, N>(dir, line, m));
-  }
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    const int ni = padn<N>(line_node<DIM, N>(dir, line, i));
-    NodeState<DIM> Li;
-    Li.rho = U[ni];
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) Li.v[d] = P[d * NDP + ni];
-    Li.p = P[Q::P * NDP + ni];
-    Li.beta = VF == VF_RANOCHA ? 0.0 : P[Q::BETA * NDP + ni];
-    Li.kin = VF == VF_CHANDRASHEKAR ? P[Q::KIN * NDP + ni] : 0.0;
-#pragma unroll
-    for (int k = i + 1; k < N; ++k) {
-      const int nk = padn<N>(line_node<DIM, N>(dir, line, k));
-      NodeState<DIM> Rk;
-      Rk.rho = U[nk];
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) Rk.v[d] = P[d * NDP + nk];
-      Rk.p = P[Q::P * NDP + nk];
-      Rk.beta = VF == VF_RANOCHA ? 0.0 : P[Q::BETA * NDP + nk];
-      Rk.kin = VF == VF_CHANDRASHEKAR ? P[Q::KIN * NDP + nk] : 0.0;
-      double nrm[DIM];
-#pragma unroll
-      for (int c = 0; c < DIM; ++c) nrm[c] = 0.5 * (ja[i][c] + ja[k][c]);
-      double f[NV];
-      volume_flux<DIM, VF>(Li, Rk, nrm, p.inv_gm1, f);
-      const double dik = p.basis.Dsplit[i][k];
-      const double dki = p.basis.Dsplit[k][i];
-#pragma unroll
-      for (int q = 0; q < NV; ++q) {
-        acc[i][q] += dik * f[q];
-        acc[k][q] += dki * f[q];
-      }
-    }
-  }
-  if constexpr (NS) {
-    // viscous weak-form volume term along the line with Dhat on the
-    // contravariant flux Ja^dir . (-F_v) (parabolic_viscous.hpp:418-466)
-    double fc[N][NV];
-#pragma unroll
-    for (int m = 0; m < N; ++m) {
-      const int nm = padn<N>(line_node<DIM, N>(dir, line, m));
-#pragma unroll
-      for (int q = 0; q < NV; ++q)
-        fc[m][q] = ja[m][0] * wv[((el * 2 + 0) * NV + q) * NDP + nm] +
-                   ja[m][1] * wv[((el * 2 + 1) * NV + q) * NDP + nm];
-    }
-#pragma unroll
-    for (int m = 0; m < N; ++m)
-#pragma unroll
-      for (int k = 0; k < N; ++k)
-#pragma unroll
-        for (int q = 0; q < NV; ++q) acc[m][q] += p.basis.Dhat[m][k] * fc[k][q];
-  }
-  if (HG) {
-    const double alpha = alpha_s[el];
-    if (fabs(alpha - 0.0) > p.atol) {
-      // volume_flux.hpp:830-841: (1 - alpha) * DG + alpha * FV
-      const double one_m = 1.0 - alpha;
-#pragma unroll
-      for (int m = 0; m < N; ++m)
-#pragma unroll
-        for (int q = 0; q < NV; ++q) acc[m][q] *= one_m;
-      // volume_flux.hpp:457-509: LLF on subcell normals along the line
-      auto node_state = [&](int m) {
-        const int nm = padn<N>(line_node<DIM, N>(dir, line, m));
-        FaceState<DIM> st;
-#pragma unroll
-        for (int q = 0; q < NV; ++q) st.u[q] = U[q * NDP + nm];
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) st.v[d] = P[d * NDP + nm];
-        st.p = P[Q::P * NDP + nm];
-        st.a2 = gamma * st.p / st.u[0];
-        return st;
-      };
-      FaceState<DIM> sl = node_state(0);
-#pragma unroll
-      for (int fi = 1; fi < N; ++fi) {
-        const FaceState<DIM> sr = node_state(fi);
-        double nrm[DIM];
-#pragma unroll
-        for (int c = 0; c < DIM; ++c)
-          nrm[c] = __ldg(M.tab.fv[dir][c] + (int64_t)I[3 + c] * (N - 1) * N + (fi - 1) * N + line);
-        double f[NV];
-        llf_flux<DIM>(sl, sr, nrm, f);
-        const double wl = alpha * p.basis.inv_w[fi - 1];
-        const double wr = alpha * p.basis.inv_w[fi];
-#pragma unroll
-        for (int q = 0; q < NV; ++q) {
-          acc[fi - 1][q] += wl * f[q];
-          acc[fi][q] -= wr * f[q];
-        }
-        sl = sr;
-      }
-    }
-  }
-  // surface fluxes at both ends of the line, lifted into the end nodes
-  // (surface_integral.hpp:35-154)
-  // Large face codes (HLLC, boundary states, viscous flux) are emitted once
-  // and called for both sides; small ones are specialised per side.
-  constexpr bool kCompactFaces = HG || SF == SF_HLLC || NS;
-  if constexpr (kCompactFaces) {
-#pragma unroll 1
-    for (int side = 0; side < 2; ++side) {
-      double f[NV];
-      element_face_flux<DIM, N, VF, SF, NS, NDP>(p, M, U, P, wv + el * 2 * NV * NDP, I, dir, side,
-                                                 line, gamma, t_stage, c0, c1, c2, f);
-      if (side == 0) {
-#pragma unroll
-        for (int q = 0; q < NV; ++q) acc[0][q] -= f[q] * p.basis.lhat_l0;
-      } else {
-#pragma unroll
-        for (int q = 0; q < NV; ++q) acc[N - 1][q] += f[q] * p.basis.lhat_rN;
-      }
-    }
-  } else {
-    double f[NV];
-    element_face_flux<DIM, N, VF, SF, NS, NDP>(p, M, U, P, wv + el * 2 * NV * NDP, I, dir, 0, line,
-                                               gamma, t_stage, c0, c1, c2, f);
-#pragma unroll
-    for (int q = 0; q < NV; ++q) acc[0][q] -= f[q] * p.basis.lhat_l0;
-    element_face_flux<DIM, N, VF, SF, NS, NDP>(p, M, U, P, wv + el * 2 * NV * NDP, I, dir, 1, line,
-                                               gamma, t_stage, c0, c1, c2, f);
-#pragma unroll
-    for (int q = 0; q < NV; ++q) acc[N - 1][q] += f[q] * p.basis.lhat_rN;
-  }
-  double* V = dv + (el * DIM + dir) * NV * NDP;
-#pragma unroll
-  for (int m = 0; m < N; ++m) {
-    const int nm = padn<N>(line_node<DIM, N>(dir, line, m));
-#pragma unroll
-    for (int q = 0; q < NV; ++q) V[q * NDP + nm] = acc[m][q];
-  }
-}
-
-// Body of the fused stage kernel; the two __global__ wrappers below differ
-// only in their launch bounds.
-template <int DIM, int N, int VF, int SF, bool HG, int EPB, int NT, bool NS, bool BATCH>
-__device__ __forceinline__ void stage_body(const StageArgs<N>& p) {
-  using S = StageShape<DIM, N, VF, SF, HG, EPB, NS>;
-  using Q = NodeSlots<DIM, VF>;
-  static_assert(!NS || (DIM == 2 && !HG), "Navier-Stokes: 2D split form only");
-  static_assert(!HG || DIM == 2, "shock capturing: 2D only");
-  constexpr int NV = S::NV, ND = S::ND, NDP = S::NDP, NF = S::NF, NFACE = S::NFACE,
-                NLINE = S::NLINE, NQ = S::NQ, NI = S::NI;
-  extern __shared__ double smem[];
-  double* us = smem;                 // [el][var][pnode]
-  double* pr = us + S::SM_U;         // [el][slot][pnode]
-  double* dv = pr + S::SM_P;         // [el][dir][var][pnode]
-  double* alpha_s = dv + S::SM_V;    // [el]
-  double* wv = alpha_s + S::SM_A;    // [el][dim][var][pnode] (NS)
-  double* vinv_s = wv + S::SM_W;     // inverse Legendre Vandermonde (HG)
-  int* info = reinterpret_cast<int*>(vinv_s + S::SM_VINV);
-
-  const int tid = threadIdx.x;
-  // Batched launches stage the block's mesh view in shared memory; single-mesh
-  // launches read it from the kernel parameters (constant bank), which keeps
-  // the table pointers out of shared-memory loads in the line loop.  The tile
-  // list and the mesh views are written by host copies only, so they are
-  // read before waiting for the previous kernel.
-  __shared__ MeshView mesh_s;
-  int e0;
-  if constexpr (BATCH) {
-    static_assert(NT >= int(sizeof(MeshView) / 8), "block narrower than the mesh view");
-    e0 = p.tile_e0[blockIdx.x];
-    copy_mesh_view(&mesh_s, p.meshes, p.tile_mesh[blockIdx.x], tid);
-  } else {
-    e0 = (int)blockIdx.x * EPB;
-  }
-  stage_dependency_sync();
-  if constexpr (BATCH) __syncthreads();
-  const MeshView& M = BATCH ? mesh_s : p.mesh;
-  const int nelem = M.nelem;
-  if (e0 >= nelem) return;
-  const int ne = min(EPB, nelem - e0);
-  const double gamma = p.gamma;
-  const double t_stage = p.t_dev ? (*p.t_dev + p.t) : p.t;
-  const int c0 = M.cells[0], c1 = M.cells[1], c2 = M.cells[2];
-
-  // ---- phase 0: element info and the contiguous u_in tile ----------------
-  for (int el = tid; el < ne; el += NT) {
-    const int e = e0 + el;
-    int ijk[3];
-    ijk[0] = e % c0;
-    ijk[1] = DIM == 2 ? e / c0 : (e / c0) % c1;
-    ijk[2] = DIM == 2 ? 0 : e / (c0 * c1);
-    int* I = info + el * NI;
-    I[0] = ijk[0];
-    I[1] = ijk[1];
-    I[2] = ijk[2];
-    if (DIM == 2) {
-      I[3] = ijk[1];
-      I[4] = ijk[0];
-      I[5] = 0;
-    } else {
-      I[3] = ijk[1] + c1 * ijk[2];
-      I[4] = ijk[0] + c0 * ijk[2];
-      I[5] = ijk[0] + c0 * ijk[1];
-    }
-    const int cells[3] = {c0, c1, c2};
-#pragma unroll
-    for (int face = 0; face < NFACE; ++face) {
-      const int dir = face >> 1, side = face & 1;
-      int pos = ijk[dir] + (side ? 1 : -1);
-      int nbr = -1;
-      if (pos < 0 || pos >= cells[dir]) {
-        if (M.periodic[dir]) pos = (pos + cells[dir]) % cells[dir];
-        else pos = -1;
-      }
-      if (pos >= 0) {
-        int q[3] = {ijk[0], ijk[1], ijk[2]};
-        q[dir] = pos;
-        nbr = DIM == 2 ? q[0] + c0 * q[1] : q[0] + c0 * (q[1] + c1 * q[2]);
-      }
-      I[6 + face] = nbr;
-    }
-  }
-  if (HG) {
-    for (int k = tid; k < N * N; k += NT) vinv_s[k] = p.basis.Vinv[k / N][k % N];
-  }
-  load_element_tile<N, NV, ND, NDP, EPB, NT>(M.u_in + (int64_t)e0 * NV * ND, us, ne, tid);
-  __syncthreads();
-
-  // ---- phase 1: node primitives, -1/J, HG alpha, -F_v -----------------
-  for (int idx = tid; idx < ne * ND; idx += NT) {
-    const int el = idx / ND, node = idx % ND;
-    const int pn = padn<N>(node);
-    double u[NV];
-#pragma unroll
-    for (int q = 0; q < NV; ++q) u[q] = us[(el * NV + q) * NDP + pn];
-    const NodeState<DIM> s = prepare_node<DIM, VF>(u, gamma);
-    double* P = pr + el * NQ * NDP + pn;
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) P[d * NDP] = s.v[d];
-    P[Q::P * NDP] = s.p;
-    if (VF != VF_RANOCHA) P[Q::BETA * NDP] = s.beta;
-    if (VF == VF_CHANDRASHEKAR) P[Q::KIN * NDP] = s.kin;
-    const int* I = info + el * NI;
-    const int in = node % N, jn = (node / N) % N, kn = DIM == 3 ? node / (N * N) : 0;
-    double jdet = __ldg(M.tab.jdiag[0] + I[0] * N + in);
-    if (DIM == 2) {
-      jdet = jdet * __ldg(M.tab.jdiag[1] + I[1] * N + jn);
-    } else {
-      jdet = jdet * (__ldg(M.tab.jdiag[1] + I[1] * N + jn) * __ldg(M.tab.jdiag[2] + I[2] * N + kn));
-    }
-    P[Q::MIJ * NDP] = -(1.0 / jdet);
-    if constexpr (NS) {
-      // -F_v at the node from the lifted gradient (parabolic_viscous.hpp:358-396)
-      double q[4], gx[4], gy[4];
-      ns_gradient_variables(u, gamma, q);
-      const double* G = p.grad + (int64_t)(e0 + el) * 4 * 2 * ND + node;
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        gx[v] = __ldg(G + (v * 2 + 0) * ND);
-        gy[v] = __ldg(G + (v * 2 + 1) * ND);
-      }
-#pragma unroll
-      for (int d = 0; d < 2; ++d) {
-        double f[4];
-        ns_neg_viscous_flux(q, gx, gy, p.mu, p.kappa, d, f);
-#pragma unroll
-        for (int v = 0; v < 4; ++v) wv[((el * 2 + d) * NV + v) * NDP + pn] = f[v];
-      }
-    }
-  }
-  if (HG) {
-    // Hennemann-Gassner alpha (indicator.hpp:337-418): node values, the two
-    // dimension-wise modal products, then the per-element sums; node-parallel
-    // with the scratch in the (not yet used) direction-contribution buffer.
-    __syncthreads();
-    double* ind = dv;                   // [el][ND]
-    double* tmp = dv + EPB * ND;        // [el][ND]
-    double* m2 = dv + 2 * EPB * ND;     // [el][ND]
-    for (int idx = tid; idx < ne * ND; idx += NT) {
-      const int el = idx / ND, node = idx % ND;
-      const int pn = padn<N>(node);
-      const double* Ue = us + el * NV * NDP;
-      ind[idx] = hg_node_value(Ue[pn], Ue[NDP + pn], Ue[2 * NDP + pn], Ue[3 * NDP + pn]);
-    }
-    __syncthreads();
-    for (int idx = tid; idx < ne * ND; idx += NT) {
-      const int el = idx / ND, node = idx % ND, j = node / N, i = node % N;
-      double r = 0.0;
-#pragma unroll
-      for (int ii = 0; ii < N; ++ii)
-        r = __dadd_rn(r, __dmul_rn(vinv_s[i * N + ii], ind[el * ND + j * N + ii]));
-      tmp[idx] = r;
-    }
-    __syncthreads();
-    for (int idx = tid; idx < ne * ND; idx += NT) {
-      const int el = idx / ND, node = idx % ND, j = node / N, i = node % N;
-      double r = 0.0;
-#pragma unroll
-      for (int jj = 0; jj < N; ++jj)
-        r = __dadd_rn(r, __dmul_rn(vinv_s[j * N + jj], tmp[el * ND + jj * N + i]));
-      m2[idx] = __dmul_rn(r, r);
-    }
-    __syncthreads();
-    for (int el = tid; el < ne; el += NT) {
-      double total, c1, c2;
-      hg_energy_sums<N>(m2 + el * ND, &total, &c1, &c2);
-      const double a = hg_alpha_from_energies(total, c1, c2, p.hg_threshold, p.hg_s,
-                                              p.alpha_min, p.alpha_max);
-      alpha_s[el] = a;
-      if (p.alpha_out) p.alpha_out[e0 + el] = a;
-    }
-  }
-  __syncthreads();
-
-  // ---- phase 2: one line per thread: end-face fluxes + volume integral ------
-  for (int idx = tid; idx < ne * NLINE; idx += NT) {
-    const int dir = idx / (ne * NF);
-    const int el = (idx / NF) % ne;
-    const int line = idx % NF;
-    if (dir == 0) {
-      process_line<0, DIM, N, VF, SF, HG, NS, NDP, NQ, NI>(p, M, us, pr, dv, alpha_s, wv, info, el,
-                                                          line, gamma, t_stage, c0, c1, c2);
-    } else if (DIM >= 2 && dir == 1) {
-      process_line<1, DIM, N, VF, SF, HG, NS, NDP, NQ, NI>(p, M, us, pr, dv, alpha_s, wv, info, el,
-                                                          line, gamma, t_stage, c0, c1, c2);
-    } else if (DIM == 3) {
-      process_line<(DIM == 3 ? 2 : 1), DIM, N, VF, SF, HG, NS, NDP, NQ, NI>(
-          p, M, us, pr, dv, alpha_s, wv, info, el, line, gamma, t_stage, c0, c1, c2);
-    }
-  }
-  __syncthreads();
-
-  // ---- phase 3: sum of directions, -1/J, SSPRK3 combination, store -------
-  bool bad = false;
-  double dacc[3] = {0.0, 0.0, 0.0};
-  const int64_t gbase = (int64_t)e0 * NV * ND;
-  for (int idx = tid; idx < ne * ND; idx += NT) {
-    const int el = idx / ND, node = idx % ND;
-    const int pn = padn<N>(node);
-    const double mij = pr[(el * NQ + Q::MIJ) * NDP + pn];
-    double vals[NV];
-#pragma unroll
-    for (int q = 0; q < NV; ++q) {
-      double du = 0.0;
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) du += dv[((el * DIM + d) * NV + q) * NDP + pn];
-      du = du * mij;
-      const int64_t gi = gbase + (int64_t)(el * NV + q) * ND + node;
-      double val = M.c * du;
-      if (p.b != 0.0) val = p.b * us[(el * NV + q) * NDP + pn] + val;
-      if (p.a != 0.0) val = p.a * M.u_n[gi] + val;
-      bad |= !isfinite(val);
-      M.out[gi] = val;
-      vals[q] = val;
-    }
-    if (p.diag) diag_add_node<DIM, N>(vals, p.basis, node, -mij, gamma, p.inv_gm1, dacc);
-  }
-  if (bad) atomicOr(p.nonfinite, 1u);
-  if constexpr (!BATCH) {
-    if (p.diag) diag_block_store<NT>(dacc, dv, p.diag + 3 * (int64_t)blockIdx.x);
-  }
-}
-
-// Fused stage kernel, register allocation left to the compiler.
-template <int DIM, int N, int VF, int SF, bool HG, int EPB, int NT, bool NS = false,
-          bool BATCH = false>
-__global__ void __launch_bounds__(NT) stage_kernel(const StageArgs<N> p) {
-  stage_body<DIM, N, VF, SF, HG, EPB, NT, NS, BATCH>(p);
-}
-
-// Same kernel with MINB resident blocks per SM requested from the register
-// allocator (a register cap of 65536 / (MINB * NT) per thread).
-template <int DIM, int N, int VF, int SF, bool HG, int EPB, int NT, bool NS, bool BATCH,
-          int MINB>
-__global__ void __launch_bounds__(NT, MINB) stage_kernel_capped(const StageArgs<N> p) {
-  stage_body<DIM, N, VF, SF, HG, EPB, NT, NS, BATCH>(p);
 }
 
 }  // namespace dgsem

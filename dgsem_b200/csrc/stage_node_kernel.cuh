@@ -1,6 +1,6 @@
 // Node-parallel form of the fused stage kernel (split form, optionally with
 // Hennemann-Gassner shock capturing in 2D; no viscous terms): the same
-// right-hand side and SSPRK3 epilogue as stage_kernel.cuh, organised for
+// right-hand side and SSPRK3 epilogue as stage_line_kernel.cuh, organised for
 // occupancy instead of minimal flux count.
 //
 // Per block: EPB elements, EPB * n^d threads.
@@ -681,7 +681,7 @@ __device__ __forceinline__ void stage_node_body(const StageArgs<N>& p, int tile 
 
   // ---- phase 1b: Hennemann-Gassner alpha per element (indicator.hpp:337-418),
   // node-parallel with the same explicitly rounded arithmetic as
-  // stage_kernel.cuh (identical alpha and troubled-cell flags); scratch in the
+  // stage_line_kernel.cuh (identical alpha and troubled-cell flags); scratch in the
   // face buffer, which is written only afterwards ------------------------------
   if constexpr (HG) {
     // two scratch arrays used in turn: node values (A) -> x pass (B) -> y
