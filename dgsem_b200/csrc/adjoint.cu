@@ -33,9 +33,9 @@ class AdjointEngineBase {
  public:
   virtual ~AdjointEngineBase() = default;
   // out = x0 X + x1 Y + b w + c (dR/du(u))^T w.  Navier-Stokes: `grad_u` is
-  // the forward BR1 gradient of u when the caller kept it from the forward
-  // stage; nullptr recomputes it into cfg.grad first.
-  virtual cudaError_t vjp(const EngineConfig& cfg, const double* u, const double* grad_u,
+  // the forward velocity gradient of u; with `fresh` it is computed into
+  // grad_u first, otherwise the caller kept it from the forward stage.
+  virtual cudaError_t vjp(const EngineConfig& cfg, const double* u, double* grad_u, bool fresh,
                           const double* w, double* out, const double* X, double x0,
                           const double* Y, double x1, double b, double c, double* xy,
                           double* qdir, cudaStream_t s) const = 0;
@@ -47,14 +47,14 @@ class AdjointEngine final : public AdjointEngineBase {
  public:
   static constexpr int EPB = (128 / (N * N)) > 0 ? (128 / (N * N)) : 1;
 
-  cudaError_t vjp(const EngineConfig& cfg, const double* u, const double* grad_u,
+  cudaError_t vjp(const EngineConfig& cfg, const double* u, double* grad_u, bool fresh,
                   const double* w, double* out, const double* X, double x0, const double* Y,
                   double x1, double b, double c, double* xy, double* qdir,
                   cudaStream_t s) const override {
     AdjArgs<N> a{};
     a.u = u;
     a.w = w;
-    a.grad = grad_u ? grad_u : cfg.grad;
+    a.grad = grad_u;
     a.xy = xy;
     a.qdir = qdir;
     a.out = out;
@@ -75,19 +75,9 @@ class AdjointEngine final : public AdjointEngineBase {
     fill_basis_const<N>(cfg.basis, &a.basis);
     const unsigned blocks = (unsigned)((cfg.nelem + EPB - 1) / EPB);
     if constexpr (NS) {
-      GradArgs<N> ga{};
-      ga.u = u;
-      ga.grad = cfg.grad;
-      for (int i = 0; i < 3; ++i) ga.cells[i] = cfg.cells[i];
-      ga.nelem = cfg.nelem;
-      ga.gamma = cfg.gamma;
-      ga.tab = cfg.tab;
-      ga.basis = a.basis;
-      ga.periodic[0] = ga.periodic[1] = 1;  // the adjoint covers periodic meshes
-      for (int f = 0; f < 4; ++f) ga.bc_kind[f] = 0;
       // programmatic dependent launches: each kernel's blocks are placed while
       // the previous one drains; griddepcontrol.wait orders the memory
-      if (!grad_u) launch_stage_kernel(br1_gradient_kernel<N, EPB>, blocks, EPB * N * N, 0, s, ga);
+      if (fresh) launch_viscous_flux<2, N>(cfg, u, nullptr, grad_u, s);
       launch_stage_kernel(adj_viscous_kernel<N, EPB>, blocks, EPB * N * N, 0, s, a);
     }
     launch_stage_kernel(adj_main_kernel<N, NS, EPB>, blocks, EPB * N * N, 0, s, a);
@@ -239,6 +229,7 @@ struct dgsem_adjoint {
   // written by the forward stages that consume them (nullptr: Euler)
   double* gseg = nullptr;
   int64_t glen = 0;
+  double* gwork = nullptr;  // velocity gradient of a standalone VJP
   double* work = nullptr;   // forward state
   double* lam = nullptr;
   double* lam2 = nullptr;
@@ -293,8 +284,8 @@ double* grad_slot(dgsem_adjoint* a, int r, int k) {
   return a->gseg ? a->gseg + ((int64_t)r * 3 + k) * a->glen : nullptr;
 }
 
-// Forward stage that keeps the BR1 gradient of its input state in `gslot`
-// (the engine writes and reads the gradient through cfg.grad).
+// Forward stage that keeps the velocity gradient of its input state in `gslot`
+// (the engine writes it through cfg.grad).
 cudaError_t fwd_stage_keep(dgsem_adjoint* a, int stage, const double* u_n, const double* u_in,
                            double* out, double t, double dt, double* gslot) {
   if (!gslot) return fwd_stage(a, stage, u_n, u_in, out, t, dt);
@@ -328,11 +319,13 @@ cudaError_t record_segment(dgsem_adjoint* a, double* state, int s0, int s1, doub
   return e;
 }
 
-cudaError_t launch_vjp(dgsem_adjoint* a, const double* u, const double* grad_u,
-                       const double* w, double* out, const double* X, double x0,
+cudaError_t launch_vjp(dgsem_adjoint* a, const double* u, double* grad_u, const double* w,
+                       double* out, const double* X, double x0,
                        const double* Y, double x1, double b, double c) {
-  a->ctx->launches += a->eng->kernels_per_vjp(grad_u == nullptr);
-  return a->eng->vjp(a->ctx->cfg, u, grad_u, w, out, X, x0, Y, x1, b, c, a->xy, a->qdir,
+  // without a kept gradient (standalone VJP) it is computed into the scratch
+  const bool fresh = grad_u == nullptr;
+  a->ctx->launches += a->eng->kernels_per_vjp(fresh);
+  return a->eng->vjp(a->ctx->cfg, u, fresh ? a->gwork : grad_u, fresh, w, out, X, x0, Y, x1, b, c, a->xy, a->qdir,
                      a->ctx->stream);
 }
 
@@ -390,7 +383,8 @@ dgsem_status dgsem_adjoint_create(dgsem_ctx* ctx, int nsteps, int checkpoint_eve
   if (a->lam2) a->lam1 = adj_alloc(a, a->len, &err);
   a->glen = ns ? nodes * 8 : 0;
   if (a->lam1 && ns) a->gseg = adj_alloc(a, (size_t)a->every * 3 * a->glen, &err);
-  if (a->lam1 && (!ns || a->gseg)) a->xy = adj_alloc(a, ns ? (size_t)nodes * 8 : 1, &err);
+  if (a->gseg) a->gwork = adj_alloc(a, a->glen, &err);
+  if (a->lam1 && (!ns || a->gwork)) a->xy = adj_alloc(a, ns ? (size_t)nodes * 8 : 1, &err);
   if (a->xy) a->qdir = adj_alloc(a, ns ? (size_t)nodes * 2 : 1, &err);
   if (a->qdir) a->partial = adj_alloc(a, (size_t)a->ke_blocks * 2, &err);
   if (a->partial) a->result = adj_alloc(a, 2, &err);

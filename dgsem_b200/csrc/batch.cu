@@ -431,6 +431,7 @@ dgsem_status dgsem_batch_create(const dgsem_mesh_desc* meshes, int n_meshes,
     c.basis = bases[g.n];
     c.nonfinite = b->flag;
     c.grad = nullptr;
+    c.visc = nullptr;
     c.elem_info = nullptr;  // batched launches take the tables from the mesh views
     c.mij = nullptr;
     for (int f = 0; f < 6; ++f) c.bc.kind[f] = 0;

@@ -383,10 +383,11 @@ dgsem_status dgsem_ctx_create(const dgsem_mesh_desc* mesh,
   ctx->tdev = ctx->staging ? device_alloc<double>(ctx, 1, &err) : nullptr;
   ctx->flag = ctx->tdev ? device_alloc<unsigned int>(ctx, 1, &err) : nullptr;
   c.grad = nullptr;
+  c.visc = nullptr;
   if (ctx->flag && is_navier_stokes(scheme->equation)) {
-    // four gradient variables x ndims directions per node
-    c.grad = device_alloc<double>(ctx, (size_t)c.nelem * 4 * nd * ctx->nodes, &err);
-    if (!c.grad) ctx->flag = nullptr;
+    // ndims directions x (ndims momentum rows and the energy row) per node
+    c.visc = device_alloc<double>(ctx, (size_t)c.nelem * nd * (nd + 1) * ctx->nodes, &err);
+    if (!c.visc) ctx->flag = nullptr;
   }
   // per-element info and -1/J per node, computed once here instead of in
   // every stage launch

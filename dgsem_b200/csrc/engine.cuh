@@ -38,7 +38,8 @@ struct EngineConfig {
   BcParams bc;
   BasisTables basis;
   unsigned int* nonfinite;  // device flag
-  double* grad;             // Navier-Stokes lifted gradient [E][4][2][n^2]
+  double* visc;             // Navier-Stokes contravariant viscous flux (br1_kernel.cuh)
+  double* grad;             // adjoint: velocity gradient written with it (may be null)
   // per-element info (node_element_info layout, 12 ints per element) and
   // -1/J per node [E][n^d], computed once per context (may be null)
   const int* elem_info;
@@ -132,9 +133,7 @@ inline StageArgs<N> stage_args_common(const EngineConfig& cfg, double a, double 
   args.hg_s = cfg.hg_s;
   args.alpha_out = alpha_out;
   args.nonfinite = cfg.nonfinite;
-  args.grad = cfg.grad;
-  args.mu = cfg.mu;
-  args.kappa = cfg.gamma / ((cfg.gamma - 1.0) * cfg.prandtl);
+  args.visc = cfg.visc;
   args.bc = cfg.bc;
   args.wait_limit_ns = cfg.wait_limit_ns;
   args.skip_tile_copy = cfg.skip_tile_copy;
@@ -200,18 +199,43 @@ void launch_stage_kernel(void (*kernel)(P...), unsigned grid, unsigned block, si
   cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
+// Contravariant viscous flux of u into `visc` (and the adjoint's velocity
+// gradient into `grad`); either output may be null.
+template <int DIM, int N>
+inline void launch_viscous_flux(const EngineConfig& cfg, const double* u, double* visc,
+                                double* grad, cudaStream_t s) {
+  using S = ViscShape<DIM, N>;
+  ViscArgs<N> a{};
+  a.u = u;
+  a.visc = visc;
+  a.grad = grad;
+  a.nelem = (int)cfg.nelem;
+  a.gamma = cfg.gamma;
+  a.mu = cfg.mu;
+  a.kappa = cfg.gamma / ((cfg.gamma - 1.0) * cfg.prandtl);
+  a.tab = cfg.tab;
+  a.info = cfg.elem_info;
+  a.mij = cfg.mij;
+  fill_basis_const<N>(cfg.basis, &a.basis);
+  for (int f = 0; f < 2 * DIM; ++f) a.bc_kind[f] = cfg.bc.kind[f];
+  const unsigned blocks = (unsigned)((cfg.nelem + S::EPB - 1) / S::EPB);
+  launch_stage_kernel(viscous_flux_kernel<DIM, N>, blocks, 32 * S::WPB, S::smem_bytes, s, a);
+}
+
+template <int DIM, int N>
+inline void set_viscous_flux_attributes() {
+  cudaFuncSetAttribute(viscous_flux_kernel<DIM, N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)ViscShape<DIM, N>::smem_bytes);
+}
+
 template <int DIM, int N, int VF, int SF, bool HG, bool NS = false>
 class Engine final : public EngineBase {
  public:
-  static constexpr int GRAD_EPB = (128 / ipow(N, DIM)) > 0 ? (128 / ipow(N, DIM)) : 1;
   static constexpr bool kBatch = !NS && !HG;
-  // the line-sweep shapes 0-2 have no viscous terms: with Navier-Stokes they
-  // run shape 3
-  static constexpr bool kLine = !NS;
 
   template <int V, bool B>
   static auto line_kernel() {
-    return stage_line_kernel<DIM, N, VF, SF, HG, B, LineLaunch<N, V>::WPB, LineLaunch<N, V>::MINB>;
+    return stage_line_kernel<DIM, N, VF, SF, HG, NS, B, LineLaunch<N, V>::WPB, LineLaunch<N, V>::MINB>;
   }
   template <int V>
   static constexpr size_t line_smem() {
@@ -224,9 +248,8 @@ class Engine final : public EngineBase {
 
   template <int V>
   static void set_attributes() {
-    if constexpr (kLine)
-      cudaFuncSetAttribute(line_kernel<V, false>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)line_smem<V>());
+    cudaFuncSetAttribute(line_kernel<V, false>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)line_smem<V>());
     if constexpr (kBatch)
       cudaFuncSetAttribute(line_kernel<V, true>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)line_smem<V>());
@@ -320,6 +343,7 @@ class Engine final : public EngineBase {
     set_attributes<0>();
     set_attributes<1>();
     set_attributes<2>();
+    if constexpr (NS) set_viscous_flux_attributes<DIM, N>();
     if constexpr (kNode) {
       const int sm = (int)NSh::smem_bytes;
       cudaFuncSetAttribute(node_kernel<false, true>(), cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
@@ -349,14 +373,10 @@ class Engine final : public EngineBase {
 
   template <int V>
   void launch(const StageArgs<N>& args, int64_t nelem, cudaStream_t s) const {
-    if constexpr (!kLine) {
-      launch_node<true>(args, nelem, s);
-    } else {
-      const int64_t blocks = (nelem + line_epb<V>() - 1) / line_epb<V>();
-      last_grid_ = blocks;
-      launch_stage_kernel(line_kernel<V, false>(), (unsigned)blocks, LineLaunch<N, V>::NT,
-                          line_smem<V>(), s, args);
-    }
+    const int64_t blocks = (nelem + line_epb<V>() - 1) / line_epb<V>();
+    last_grid_ = blocks;
+    launch_stage_kernel(line_kernel<V, false>(), (unsigned)blocks, LineLaunch<N, V>::NT,
+                        line_smem<V>(), s, args);
   }
 
   cudaError_t stage(const EngineConfig& cfg, const double* u_n,
@@ -377,25 +397,7 @@ class Engine final : public EngineBase {
     args.mesh.tab = cfg.tab;
     args.mesh.info = cfg.elem_info;
     args.mesh.mij = cfg.mij;
-    if constexpr (NS) {
-      GradArgs<N> ga{};
-      ga.u = u_in;
-      ga.grad = cfg.grad;
-      for (int i = 0; i < 3; ++i) ga.cells[i] = cfg.cells[i];
-      ga.nelem = cfg.nelem;
-      ga.gamma = cfg.gamma;
-      ga.tab = cfg.tab;
-      ga.basis = args.basis;
-      for (int d = 0; d < DIM; ++d) ga.periodic[d] = cfg.periodic[d];
-      for (int f = 0; f < 2 * DIM; ++f) ga.bc_kind[f] = cfg.bc.kind[f];
-      const int64_t gblocks = (cfg.nelem + GRAD_EPB - 1) / GRAD_EPB;
-      if constexpr (DIM == 2)
-        launch_stage_kernel(br1_gradient_kernel<N, GRAD_EPB>, (unsigned)gblocks, GRAD_EPB * N * N,
-                            0, s, ga);
-      else
-        launch_stage_kernel(br1_gradient_kernel_3d<N, GRAD_EPB>, (unsigned)gblocks,
-                            GRAD_EPB * N * N * N, 0, s, ga);
-    }
+    if constexpr (NS) launch_viscous_flux<DIM, N>(cfg, u_in, cfg.visc, cfg.grad, s);
     switch (variant_) {
       case 1: launch<1>(args, cfg.nelem, s); break;
       case 2: launch<2>(args, cfg.nelem, s); break;
@@ -454,18 +456,20 @@ class Engine final : public EngineBase {
   int elements_per_block() const override {
     if constexpr (kNode2)
       if (variant_ == 6) return Node2Launch<N>::EPB;
-    if (variant_ >= 3 || !kLine) return NL::EPB;
-    return variant_ == 2 ? line_epb<2>() : line_epb<0>();
+    if (variant_ >= 3) return NL::EPB;
+    return variant_ == 2 ? line_epb<2>() : variant_ == 1 ? line_epb<1>() : line_epb<0>();
   }
   int threads_per_block() const override {
-    if (variant_ >= 3 || !kLine) return NL::NT;
-    return variant_ == 2 ? LineLaunch<N, 2>::NT : LineLaunch<N, 0>::NT;
+    if (variant_ >= 3) return NL::NT;
+    return variant_ == 2 ? LineLaunch<N, 2>::NT
+           : variant_ == 1 ? LineLaunch<N, 1>::NT
+                           : LineLaunch<N, 0>::NT;
   }
   size_t smem_bytes() const override {
     if constexpr (kNode2)
       if (variant_ == 6) return Node2Shape<N, VF>::smem_bytes;
-    if (variant_ >= 3 || !kLine) return NSh::smem_bytes;
-    return variant_ == 2 ? line_smem<2>() : line_smem<0>();
+    if (variant_ >= 3) return NSh::smem_bytes;
+    return variant_ == 2 ? line_smem<2>() : variant_ == 1 ? line_smem<1>() : line_smem<0>();
   }
   void set_variant(int v) override { variant_ = (v >= 0 && v < num_variants()) ? v : 0; }
   int variant() const override { return variant_; }

@@ -108,8 +108,7 @@ struct StageArgs {
   double alpha_max, alpha_min, atol, hg_threshold, hg_s;
   double* alpha_out;       // optional per-element alpha
   unsigned int* nonfinite;
-  const double* grad;      // Navier-Stokes lifted gradient [E][4][2][ND]
-  double mu, kappa;
+  const double* visc;      // Navier-Stokes contravariant viscous flux (br1_kernel.cuh)
   BcParams bc;
   BasisConst<N> basis;
   // Failure-path testing only (both 0 in normal use): bound of the tile-copy
@@ -535,18 +534,6 @@ __device__ __forceinline__ void load_element_tile(const double* src, double* us,
   t.store(src, us, ne, tid);
 }
 
-// Navier-Stokes pieces used by the stage kernel (defined in br1_kernel.cuh).
-__device__ __forceinline__ void ns_gradient_variables(const double* u, double gamma,
-                                                      double* q);
-__device__ __forceinline__ void ns_neg_viscous_flux(const double* q, const double* gx,
-                                                    const double* gy, double mu,
-                                                    double kappa, int dim, double* f);
-__device__ __forceinline__ void ns_gradient_variables_3d(const double* u, double gamma,
-                                                         double* q);
-__device__ __forceinline__ void ns_neg_viscous_flux_3d(const double* q, const double (*g)[4],
-                                                       double mu, double kappa, int dim,
-                                                       double* f);
-
 // Element index over the axes != c of the element whose coordinate along
 // `dir` is replaced by `pos` (the neighbour across a face of direction dir).
 template <int DIM>
@@ -567,12 +554,11 @@ __device__ __forceinline__ int eidx_other_shift(const int* I, int c, int dir, in
 template <int DIM, int N, int VF, int SF, bool NS, int NDP>
 __device__ __forceinline__ void element_face_flux_state(
     const StageArgs<N>& p, const MeshView& M, const FaceState<DIM>& so, const double* us_el,
-    const double* wv_el, const int* I, int dir, int side, int line, double gamma,
-    double t_stage, int c0, int c1, int c2, double* f) {
+    int e_own, const int* I, int dir, int side, int line, double gamma, double t_stage, int c0,
+    int c1, int c2, double* f) {
   constexpr int NV = DIM + 2, ND = ipow(N, DIM);
   constexpr bool PAD = NDP != ND;
   const int own_node = line_node<DIM, N>(dir, line, side ? N - 1 : 0);
-  const int opn = padn<N, PAD>(own_node);
   const int face = 2 * dir + side;
   const int en = I[6 + face];
   // the state on the far side of the face (neighbour trace or boundary
@@ -630,61 +616,24 @@ __device__ __forceinline__ void element_face_flux_state(
   } else {
     surface_flux<DIM, SF>(sx, so, nrm, gamma, f);
   }
-  if constexpr (NS && DIM == 3) {
-    // 3D periodic meshes: the one-sided viscous interface flux -F_v . n of the
-    // high-side (primary) element at its low-face node
-    // (parabolic_viscous.hpp:570-585), lifted like the inviscid flux
-    double w[3][5];
-    if (side) {
-      double q[5], g[3][4];
-      ns_gradient_variables_3d(ux, gamma, q);
-      const double* G = p.grad + (int64_t)en * 4 * 3 * ND + nb_node;
-#pragma unroll
-      for (int v = 0; v < 4; ++v)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) g[d][v] = __ldg(G + (v * 3 + d) * ND);
-#pragma unroll
-      for (int d = 0; d < 3; ++d) ns_neg_viscous_flux_3d(q, g, p.mu, p.kappa, d, w[d]);
-    } else {
-#pragma unroll
-      for (int d = 0; d < 3; ++d)
-#pragma unroll
-        for (int v = 0; v < 5; ++v) w[d][v] = wv_el[(d * NV + v) * NDP + opn];
-    }
-#pragma unroll
-    for (int v = 0; v < 5; ++v) f[v] += w[0][v] * nrm[0] + w[1][v] * nrm[1] + w[2][v] * nrm[2];
-  } else if constexpr (NS) {
+  if constexpr (NS) {
+    // the one-sided viscous interface flux -F_v . n of the high-side (primary)
+    // element at its low-face node (parabolic_viscous.hpp:570-585) is its
+    // contravariant viscous flux there (br1_kernel.cuh); lifted with the same
+    // factors as the inviscid flux
+    constexpr int NQ = DIM + 1;
+    const int eh = en >= 0 && side ? en : e_own;
+    const int node = en >= 0 ? line_node<DIM, N>(dir, line, 0) : own_node;
+    const double* V = p.visc + ((int64_t)eh * DIM + dir) * (NQ * ND) + node;
     if (en >= 0) {
-      // one-sided viscous interface flux: -F_v . n of the high-side (primary)
-      // element at its low-face node (parabolic_viscous.hpp:570-585), lifted
-      // with the same factors as the inviscid flux
-      double w[2][4];
-      if (side) {
-        double q[4], gx[4], gy[4];
-        ns_gradient_variables(ux, gamma, q);
-        const double* G = p.grad + (int64_t)en * 4 * 2 * ND + nb_node;
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          gx[v] = __ldg(G + (v * 2 + 0) * ND);
-          gy[v] = __ldg(G + (v * 2 + 1) * ND);
-        }
-        ns_neg_viscous_flux(q, gx, gy, p.mu, p.kappa, 0, w[0]);
-        ns_neg_viscous_flux(q, gx, gy, p.mu, p.kappa, 1, w[1]);
-      } else {
-#pragma unroll
-        for (int d = 0; d < 2; ++d)
-#pragma unroll
-          for (int v = 0; v < 4; ++v) w[d][v] = wv_el[(d * NV + v) * NDP + opn];
-      }
-#pragma unroll
-      for (int v = 0; v < 4; ++v) f[v] += w[0][v] * nrm[0] + w[1][v] * nrm[1];
+      for (int r = 0; r < NQ; ++r) f[1 + r] += __ldg(V + r * ND);
     } else if (p.bc.kind[face] == BC_NS_NOSLIP_ADIABATIC_WALL) {
       // NSNoSlipAdiabaticWallBC::apply_viscous_device (navier_stokes_wall_
-      // boundary.hpp:101-131): the inner -F_v . n on the momentum, no mass
-      // or energy flux (adiabatic); the slip wall adds nothing
+      // boundary.hpp:101-131): the inner -F_v . n on the momentum, no mass or
+      // energy flux (adiabatic); the slip wall adds nothing
 #pragma unroll
-      for (int v = 1; v < 3; ++v)
-        f[v] += wv_el[(0 * NV + v) * NDP + opn] * nrm[0] + wv_el[(1 * NV + v) * NDP + opn] * nrm[1];
+      for (int r = 0; r < DIM; ++r) f[1 + r] += __ldg(V + r * ND);
     }
   }
 }

@@ -1,5 +1,6 @@
 // Line-sweep form of the fused stage kernel (launch shapes 0-2): split form,
-// optionally with Hennemann-Gassner shock capturing, 2D and 3D, the same
+// optionally with Hennemann-Gassner shock capturing and with the viscous terms
+// (br1_kernel.cuh), 2D and 3D, the same
 // right-hand side and SSPRK3 epilogue as stage_node_kernel.cuh.
 //
 // One warp works on EPW = 32 / n^(d-1) whole elements and on nothing else:
@@ -100,24 +101,27 @@ struct LinePos {
   int off[N];
   int first, stride;
 
-  __device__ __forceinline__ void set(int dir, int el, int line) {
+  static __device__ __forceinline__ int slot(int dir, int el, int line, int m) {
     using G = LineGeo<DIM, N>;
+    const int lo = line % N, hi = DIM == 3 ? line / N : 0;
+    const int i = dir == 0 ? m : lo;
+    const int j = dir == 0 ? lo : dir == 1 ? m : hi;
+    const int k = dir == 2 ? m : hi;
+    if constexpr (G::SWZ) {
+      const int kk = DIM == 2 ? (el & 3) : k;
+      const int base = DIM == 2 ? 16 * el : 64 * el + 16 * k;
+      return base + 4 * (j ^ kk) + (i ^ (2 * (kk & 1)));
+    } else {
+      return el * G::PL + (j + N * k) * G::LS + i;
+    }
+  }
+
+  __device__ __forceinline__ void set(int dir, int el, int line) {
     const int lo = line % N, hi = DIM == 3 ? line / N : 0;
     stride = dir == 0 ? 1 : dir == 1 ? N : N * N;
     first = dir == 0 ? N * line : dir == 1 ? lo + N * N * hi : line;
 #pragma unroll
-    for (int m = 0; m < N; ++m) {
-      const int i = dir == 0 ? m : lo;
-      const int j = dir == 0 ? lo : dir == 1 ? m : hi;
-      const int k = dir == 2 ? m : hi;
-      if constexpr (G::SWZ) {
-        const int kk = DIM == 2 ? (el & 3) : k;
-        const int base = DIM == 2 ? 16 * el : 64 * el + 16 * k;
-        off[m] = base + 4 * (j ^ kk) + (i ^ (2 * (kk & 1)));
-      } else {
-        off[m] = el * G::PL + (j + N * k) * G::LS + i;
-      }
-    }
+    for (int m = 0; m < N; ++m) off[m] = slot(dir, el, line, m);
   }
 };
 
@@ -457,7 +461,7 @@ __device__ __forceinline__ void line_volume_general(const StageArgs<N>& p, const
 
 // One direction of a lane's line; its contribution is added to R (FIRST:
 // written), and left in acc for the last direction at odd n.
-template <int DIM, int N, int VF, int SF, bool HG, bool XL>
+template <int DIM, int N, int VF, int SF, bool HG, bool NS, bool XL>
 __device__ __forceinline__ void line_sweep(const StageArgs<N>& p, const MeshView& M,
                                            const LineElement<DIM>& E, int dir, int el, int line,
                                            const double* P, double* R, double alpha,
@@ -703,6 +707,46 @@ __device__ __forceinline__ void line_sweep(const StageArgs<N>& p, const MeshView
     face(1);
   }
 
+  if constexpr (NS) {
+    // viscous terms, outside the shock-capturing blend (the reference adds
+    // the parabolic terms separately, structured_solver.hpp:437-480): Dhat
+    // product of the contravariant flux along the line (parabolic_viscous.hpp:
+    // 398-466) and the one-sided interface fluxes of the high-side elements,
+    // the line's own at its low end (br1_kernel.cuh)
+    constexpr int NQ = DIM + 1;
+    const double* V = p.visc + ((int64_t)E.e * DIM + dir) * (NQ * ND) + pos.first;
+    const double* Vn = p.visc + ((int64_t)max(nb[1], 0) * DIM + dir) * (NQ * ND) + pos.first;
+    bool lo = true, hi = true;
+    if (DIM == 2 && (nb[0] | nb[1]) < 0) {
+      // no-slip walls: the inner flux on the momentum rows; slip walls: none
+      lo = nb[0] >= 0 || p.bc.kind[2 * dir] == BC_NS_NOSLIP_ADIABATIC_WALL;
+      hi = nb[1] >= 0 || p.bc.kind[2 * dir + 1] == BC_NS_NOSLIP_ADIABATIC_WALL;
+    }
+#pragma unroll
+    for (int r = 0; r < NQ; ++r) {
+      double w[N];
+      if constexpr (XL) {
+        load_xline<N, true>(V + r * ND, w);
+      } else {
+#pragma unroll
+        for (int m = 0; m < N; ++m) w[m] = __ldg(V + r * ND + m * pos.stride);
+      }
+      double wl = w[0], wh = __ldg(Vn + r * ND);
+      if constexpr (DIM == 2) {
+        wh = nb[1] >= 0 ? wh : w[N - 1];
+        wl = !lo || (nb[0] < 0 && r == DIM) ? 0.0 : wl;
+        wh = !hi || (nb[1] < 0 && r == DIM) ? 0.0 : wh;
+      }
+#pragma unroll
+      for (int m = 0; m < N; ++m)
+#pragma unroll
+        for (int k = 0; k < N; ++k)
+          acc[m][1 + r] = __fma_rn(p.basis.Dhat[m][k], w[k], acc[m][1 + r]);
+      acc[0][1 + r] = __fma_rn(-wl, p.basis.lhat_l0, acc[0][1 + r]);
+      acc[N - 1][1 + r] = __fma_rn(wh, p.basis.lhat_rN, acc[N - 1][1 + r]);
+    }
+  }
+
   // add to R
   const bool read = dir > 0 || (VF != VF_KENNEDY_GRUBER && outside);
 #pragma unroll
@@ -801,7 +845,7 @@ __device__ __forceinline__ double line_alpha(const StageArgs<N>& p, double* S, i
   return alpha;
 }
 
-template <int DIM, int N, int VF, int SF, bool HG, bool BATCH, int WPB>
+template <int DIM, int N, int VF, int SF, bool HG, bool NS, bool BATCH, int WPB>
 __device__ __forceinline__ void stage_line_body(const StageArgs<N>& p) {
   using G = LineGeo<DIM, N>;
   using K = LineSlots<DIM, VF>;
@@ -910,18 +954,18 @@ __device__ __forceinline__ void stage_line_body(const StageArgs<N>& p) {
     for (int dir = 0; dir < DIM; ++dir) {
       __syncwarp();
       if (act)
-        line_sweep<DIM, N, VF, SF, HG, false>(p, M, E, dir, el, line, P, R, alpha, t_stage, acc,
+        line_sweep<DIM, N, VF, SF, HG, NS, false>(p, M, E, dir, el, line, P, R, alpha, t_stage, acc,
                                               pos);
     }
   } else {
     __syncwarp();
     if (act)
-      line_sweep<DIM, N, VF, SF, HG, true>(p, M, E, 0, el, line, P, R, alpha, t_stage, acc, pos);
+      line_sweep<DIM, N, VF, SF, HG, NS, true>(p, M, E, 0, el, line, P, R, alpha, t_stage, acc, pos);
 #pragma unroll
     for (int dir = 1; dir < DIM; ++dir) {
       __syncwarp();
       if (act)
-        line_sweep<DIM, N, VF, SF, HG, false>(p, M, E, dir, el, line, P, R, alpha, t_stage, acc,
+        line_sweep<DIM, N, VF, SF, HG, NS, false>(p, M, E, dir, el, line, P, R, alpha, t_stage, acc,
                                               pos);
     }
   }
@@ -1011,9 +1055,9 @@ __device__ __forceinline__ void stage_line_body(const StageArgs<N>& p) {
 }
 
 // MINB resident blocks per SM are requested from the register allocator.
-template <int DIM, int N, int VF, int SF, bool HG, bool BATCH, int WPB, int MINB>
+template <int DIM, int N, int VF, int SF, bool HG, bool NS, bool BATCH, int WPB, int MINB>
 __global__ void __launch_bounds__(32 * WPB, MINB) stage_line_kernel(const StageArgs<N> p) {
-  stage_line_body<DIM, N, VF, SF, HG, BATCH, WPB>(p);
+  stage_line_body<DIM, N, VF, SF, HG, NS, BATCH, WPB>(p);
 }
 
 }  // namespace dgsem

@@ -133,7 +133,7 @@ __device__ __forceinline__ void stage_node2_body(const StageArgs<N>& p) {
   constexpr int NV = S::NV, ND = S::ND, NDP = S::NDP, NF = S::NF, NFACE = S::NFACE,
                 NQ = S::NQ, NI = S::NI;
   static_assert(NDP == ND && !S::XCHG && S::NT == 2 * NT, "shape");
-  static_assert(S::SM_A == 0 && S::SM_VINV == 0 && S::SM_X == 0 && S::SM_W == 0, "layout");
+  static_assert(S::SM_A == 0 && S::SM_VINV == 0 && S::SM_X == 0, "layout");
   extern __shared__ __align__(128) double smem_node2[];
   double* us = smem_node2;     // [el][var][node]
   double* pr = us + S::SM_U;   // [el][slot][node]
@@ -217,7 +217,7 @@ __device__ __forceinline__ void stage_node2_body(const StageArgs<N>& p) {
   __syncthreads();
 
   // ---- phase 2a: face fluxes ---------------------------------------------
-  node_face_tasks<DIM, N, VF, SF, false, NDP, NT, NQ, NI>(p, M, us, pr, nullptr, info, sf, ne,
+  node_face_tasks<DIM, N, VF, SF, false, NDP, NT, NQ, NI>(p, M, us, pr, info, sf, e0, ne,
                                                           tid, gamma, t_stage, c0, c1, c2);
 
   // ---- phase 2b: volume term of both nodes -------------------------------

@@ -87,10 +87,8 @@ struct NodeShape {
   // smem_bytes_base and leave the rest of the SM's storage to L1
   static constexpr int SM_N = (NV * ND) % 2 == 0 ? EPB * NV * ND : 0;
   static constexpr int NT = EPB * ND;
-  // Navier-Stokes: -F_v per node [el][dim][var][node]
-  static constexpr int SM_W = NS ? EPB * DIM * NV * ND : 0;
   static constexpr size_t smem_bytes_base =
-      sizeof(double) * (SM_U + SM_P + SM_F + SM_A + SM_VINV + SM_X + SM_W) +
+      sizeof(double) * (SM_U + SM_P + SM_F + SM_A + SM_VINV + SM_X) +
       sizeof(int) * EPB * NI;
   static constexpr size_t off_n_bytes = (smem_bytes_base + 15) / 16 * 16;
   static constexpr size_t smem_bytes = off_n_bytes + sizeof(double) * SM_N;
@@ -481,8 +479,8 @@ __device__ __forceinline__ void node_lift(const double* sf_el, int node, double 
 template <int DIM, int N, int VF, int SF, bool NS, int NDP, int NT, int NQ, int NI>
 __device__ __forceinline__ void node_face_tasks(const StageArgs<N>& p, const MeshView& M,
                                                 const double* us, const double* pr,
-                                                const double* wv, const int* info, double* sf,
-                                                int ne, int tid, double gamma, double t_stage,
+                                                const int* info, double* sf, int e0, int ne,
+                                                int tid, double gamma, double t_stage,
                                                 int c0, int c1, int c2) {
   using K = NodeKernelSlots<DIM, VF>;
   constexpr int NV = DIM + 2, ND = ipow(N, DIM), NF = ipow(N, DIM - 1), NFACE = 2 * DIM;
@@ -502,7 +500,7 @@ __device__ __forceinline__ void node_face_tasks(const StageArgs<N>& p, const Mes
     so.a2 = P[K::A * NDP + opn];
     double f[NV];
     element_face_flux_state<DIM, N, VF, SF, NS, NDP>(p, M, so, U,
-                                                     NS ? wv + fe * DIM * NV * ND : nullptr, I,
+                                                     e0 + fe, I,
                                                      dir, side, fn, gamma, t_stage, c0, c1, c2,
                                                      f);
     double* F = sf + ((fe * NFACE + face) * NF + fn) * NV;
@@ -546,8 +544,7 @@ __device__ __forceinline__ void stage_node_body(const StageArgs<N>& p, int tile 
   double* alpha_s = sf + S::SM_F;          // [el] (shock capturing)
   double* vinv_s = alpha_s + S::SM_A;      // [N][N] (shock capturing)
   double* xbuf = vinv_s + S::SM_VINV;      // volume-term exchange
-  double* wv = xbuf + S::SM_X;             // Navier-Stokes -F_v [el][dim][var][node]
-  int* info = reinterpret_cast<int*>(wv + S::SM_W);
+  int* info = reinterpret_cast<int*>(xbuf + S::SM_X);
   // [el][var][node] u_n tile (bulk-copy target; present when p.a != 0)
   double* stage_n = reinterpret_cast<double*>(reinterpret_cast<char*>(smem_node) + S::off_n_bytes);
 
@@ -623,44 +620,10 @@ __device__ __forceinline__ void stage_node_body(const StageArgs<N>& p, int tile 
   if constexpr (HG) {
     for (int k = tid; k < N * N; k += NT) vinv_s[k] = p.basis.Vinv[k / N][k % N];
   }
-  // node data, squared sound speed and -1/J (and -F_v with viscous terms)
+  // node data, squared sound speed and -1/J
   auto node_data = [&](const double* u) {
     node_prepare<DIM, N, VF, NDP>(M, u, gamma, info + el * NI, node, pr + el * NQ * NDP + pn,
                                   own_node ? &mij_node : nullptr);
-    if constexpr (NS && DIM == 3) {
-      // -F_v at the node from the lifted gradient (parabolic_viscous.hpp:358-396)
-      double q[5], g[3][4];
-      ns_gradient_variables_3d(u, gamma, q);
-      const double* G = p.grad + (int64_t)(e0 + el) * 4 * 3 * ND + node;
-#pragma unroll
-      for (int v = 0; v < 4; ++v)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) g[d][v] = __ldg(G + (v * 3 + d) * ND);
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        double f[5];
-        ns_neg_viscous_flux_3d(q, g, p.mu, p.kappa, d, f);
-#pragma unroll
-        for (int v = 0; v < 5; ++v) wv[((el * 3 + d) * NV + v) * ND + node] = f[v];
-      }
-    } else if constexpr (NS) {
-      // -F_v at the node from the lifted gradient (parabolic_viscous.hpp:358-396)
-      double q[4], gx[4], gy[4];
-      ns_gradient_variables(u, gamma, q);
-      const double* G = p.grad + (int64_t)(e0 + el) * 4 * 2 * ND + node;
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        gx[v] = __ldg(G + (v * 2 + 0) * ND);
-        gy[v] = __ldg(G + (v * 2 + 1) * ND);
-      }
-#pragma unroll
-      for (int d = 0; d < 2; ++d) {
-        double f[4];
-        ns_neg_viscous_flux(q, gx, gy, p.mu, p.kappa, d, f);
-#pragma unroll
-        for (int v = 0; v < 4; ++v) wv[((el * 2 + d) * NV + v) * ND + node] = f[v];
-      }
-    }
   };
   if (own_node) {
     if (active) {
@@ -744,7 +707,7 @@ __device__ __forceinline__ void stage_node_body(const StageArgs<N>& p, int tile 
 
   // ---- phase 2a: face fluxes, one task per (element, face, face node) ------
   if (worker)
-    node_face_tasks<DIM, N, VF, SF, NS, NDP, NT, NQ, NI>(p, M, us, pr, wv, info, sf, ne, tid,
+    node_face_tasks<DIM, N, VF, SF, NS, NDP, NT, NQ, NI>(p, M, us, pr, info, sf, e0, ne, tid,
                                                          gamma, t_stage, c0, c1, c2);
 
   // ---- phase 2b: volume term, one thread per node --------------------------
@@ -798,49 +761,19 @@ __device__ __forceinline__ void stage_node_body(const StageArgs<N>& p, int tile 
   // separately, structured_solver.hpp:437-480)
   if constexpr (NS) {
     if (active) {
-      const int ev = el;
-      const int* I = info + el * NI;
-      if constexpr (NS && DIM == 3) {
-        // viscous weak-form volume term sum_k Dhat(m, k) Ja^dir(k) . (-F_v)(k)
-        // along each line through the node (parabolic_viscous.hpp:398-469)
-        const double* W = wv + ev * 3 * NV * ND;
+      // viscous weak-form volume term sum_k Dhat(m, k) Ja^dir(k) . (-F_v)(k)
+      // along each line through the node (parabolic_viscous.hpp:418-466)
+      const double* W = p.visc + (int64_t)(e0 + el) * (DIM * (DIM + 1) * ND);
 #pragma unroll
-        for (int dir = 0; dir < 3; ++dir) {
-          const int m = dir == 0 ? node % N : dir == 1 ? (node / N) % N : node / (N * N);
-          const int stride = dir == 0 ? 1 : dir == 1 ? N : N * N;
-          const double* j0 = M.tab.ja[dir][0] + (int64_t)I[3] * ND;
-          const double* j1 = M.tab.ja[dir][1] + (int64_t)I[4] * ND;
-          const double* j2 = M.tab.ja[dir][2] + (int64_t)I[5] * ND;
+      for (int dir = 0; dir < DIM; ++dir) {
+        const int m = dir == 0 ? node % N : dir == 1 ? (node / N) % N : node / (N * N);
+        const int stride = dir == 0 ? 1 : dir == 1 ? N : N * N;
 #pragma unroll
-          for (int k = 0; k < N; ++k) {
-            const int nk = node + (k - m) * stride;
-            const double a0 = __ldg(j0 + nk), a1 = __ldg(j1 + nk), a2 = __ldg(j2 + nk);
-            const double dmk = p.basis.Dhat[m][k];
+        for (int k = 0; k < N; ++k) {
+          const double dmk = p.basis.Dhat[m][k];
 #pragma unroll
-            for (int q = 0; q < NV; ++q)
-              acc[q] += dmk * (a0 * W[(0 * NV + q) * ND + nk] + a1 * W[(1 * NV + q) * ND + nk] +
-                               a2 * W[(2 * NV + q) * ND + nk]);
-          }
-        }
-      } else if constexpr (NS) {
-        // viscous weak-form volume term sum_k Dhat(m, k) Ja^dir(k) . (-F_v)(k)
-        // along each line through the node (parabolic_viscous.hpp:418-466)
-        const double* W = wv + ev * 2 * NV * ND;
-#pragma unroll
-        for (int dir = 0; dir < 2; ++dir) {
-          const int m = dir == 0 ? node % N : node / N;
-          const int stride = dir == 0 ? 1 : N;
-          const double* j0 = M.tab.ja[dir][0] + (int64_t)I[3] * ND;
-          const double* j1 = M.tab.ja[dir][1] + (int64_t)I[4] * ND;
-#pragma unroll
-          for (int k = 0; k < N; ++k) {
-            const int nk = node + (k - m) * stride;
-            const double a0 = __ldg(j0 + nk), a1 = __ldg(j1 + nk);
-            const double dmk = p.basis.Dhat[m][k];
-#pragma unroll
-            for (int q = 0; q < NV; ++q)
-              acc[q] += dmk * (a0 * W[(0 * NV + q) * ND + nk] + a1 * W[(1 * NV + q) * ND + nk]);
-          }
+          for (int r = 0; r <= DIM; ++r)
+            acc[1 + r] += dmk * __ldg(W + (dir * (DIM + 1) + r) * ND + node + (k - m) * stride);
         }
       }
     }

@@ -131,7 +131,7 @@ __device__ __forceinline__ void stage_pipe_body(const StageArgs<N>& p, int ntile
       request(&bar_in, stage_in, M.u_in, t + gridDim.x);
 
     // ---- phase 2a: face fluxes ---------------------------------------------
-    node_face_tasks<DIM, N, VF, SF, false, NDP, NT, NQ, NI>(p, M, us, pr, nullptr, info, sf, ne,
+    node_face_tasks<DIM, N, VF, SF, false, NDP, NT, NQ, NI>(p, M, us, pr, info, sf, e0, ne,
                                                             tid, gamma, t_stage, c0, c1, c2);
 
     // ---- phase 2b: volume term ---------------------------------------------
