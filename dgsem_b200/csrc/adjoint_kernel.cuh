@@ -58,7 +58,7 @@ __device__ __forceinline__ double adj_ja(const DeviceTables& t, int a, int c, in
 
 template <int N>
 __device__ __forceinline__ double adj_inv_j(const DeviceTables& t, int ie, int je, int node) {
-  return 1.0 / (__ldg(t.jdiag[0] + ie * N + node % N) * __ldg(t.jdiag[1] + je * N + node / N));
+  return recip(__ldg(t.jdiag[0] + ie * N + node % N) * __ldg(t.jdiag[1] + je * N + node / N));
 }
 
 // ---- derivatives of the logarithmic mean (same branch rule as chandrashekar_means);
@@ -162,10 +162,10 @@ __device__ __forceinline__ void llf_vjp(const FaceState<2>& L, const FaceState<2
                                         double gamma, double* ub) {
   const double vnL = L.v[0] * n[0] + L.v[1] * n[1];
   const double vnR = R.v[0] * n[0] + R.v[1] * n[1];
-  const double sn = sqrt(n[0] * n[0] + n[1] * n[1]);
+  const double sn = root(n[0] * n[0] + n[1] * n[1]);
   // sound speeds from the squared ones the forward stores; lambda is the
   // forward's max|v.n| + sqrt(max(a^2) |n|^2) = max|v.n| + max(a) |n|
-  const double aL = sqrt(L.a2), aR = sqrt(R.a2);
+  const double aL = root(L.a2), aR = root(R.a2);
   const double lam = fmax(fabs(vnL), fabs(vnR)) + fmax(aL, aR) * sn;
   const FaceState<2>& O = own_left ? L : R;
   const double vnO = own_left ? vnL : vnR;
@@ -462,7 +462,7 @@ __global__ void __launch_bounds__(EPB* N* N) adj_main_kernel(const AdjArgs<N> p)
     double qv[4];
     ns_gradient_variables(u, p.gamma, qv);
     const double T = qv[3];
-    const double iu = 1.0 / u[0];
+    const double iu = recip(u[0]);
     const double rbq = qb[0] - qb[3] * T * iu;
     const double vbq[2] = {qb[1], qb[2]};
     prim_to_cons_vjp(u, gm1, rbq, vbq, qb[3] * iu, ub, iu);

@@ -32,7 +32,7 @@ namespace dgsem {
 __device__ __forceinline__ void ns_gradient_variables(const double* u, double gamma,
                                                       double* q) {
   const double rho = u[0];
-  const double inv_rho = 1.0 / rho;
+  const double inv_rho = recip(rho);
   const double v1 = u[1] * inv_rho;
   const double v2 = u[2] * inv_rho;
   const double p = (gamma - 1.0) * (u[3] - 0.5 * (u[1] * u[1] + u[2] * u[2]) * inv_rho);
