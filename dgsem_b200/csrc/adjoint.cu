@@ -80,7 +80,8 @@ class AdjointEngine final : public AdjointEngineBase {
       if (fresh) launch_viscous_flux<2, N>(cfg, u, nullptr, grad_u, s);
       launch_stage_kernel(adj_viscous_kernel<N, EPB>, blocks, EPB * N * N, 0, s, a);
     }
-    launch_stage_kernel(adj_main_kernel<N, NS, EPB>, blocks, EPB * N * N, 0, s, a);
+    launch_stage_kernel(adj_main_kernel<N, NS, EPB>, blocks, 2 * AdjMainShape<N, EPB>::HALF, 0, s,
+                        a);
     return cudaGetLastError();
   }
   int kernels_per_vjp(bool with_gradient) const override {

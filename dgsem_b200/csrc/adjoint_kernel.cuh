@@ -10,7 +10,8 @@
 //
 // Notation: w_hat = -(1/J) w per node (the cotangent of the unscaled du).
 //
-// Two kernels, one thread per node, EPB elements per block:
+// Two kernels, EPB elements per block, one thread per node (viscous) and one
+// per node and direction (main):
 //   adj_viscous_kernel (Navier-Stokes only): cotangent of the stored -F_v
 //     (transposed Dhat volume term and one-sided interface flux), then of the
 //     lifted gradient G; writes per node X~ = sum_d Ja^0_d G~_d / J and
@@ -305,149 +306,142 @@ __global__ void __launch_bounds__(EPB* N* N) adj_viscous_kernel(const AdjArgs<N>
 }
 
 // ---- inviscid cotangents, transposed BR1, chain rule, epilogue -------------
+// Two threads per node, one per direction (the block's first half of whole
+// warps takes x, the second y): a node's 2 (n - 1) partners, its faces and
+// its Dhat sums are one dependent chain of about 3 700 instructions at n = 5,
+// and the meshes an adjoint runs on leave the GPU mostly idle, so the chain's
+// length is the kernel's time: 32 x 32, n = 5, gradient through 40 steps 4310 ->
+// 3945 us.  The y half hands its 13 sums to the x half.
+template <int N, int EPB>
+struct AdjMainShape {
+  static constexpr int NT = EPB * N * N;            // nodes of a block
+  static constexpr int HALF = (NT + 31) / 32 * 32;  // threads per direction
+};
+
 template <int N, bool NS, int EPB>
-__global__ void __launch_bounds__(EPB* N* N) adj_main_kernel(const AdjArgs<N> p) {
+__global__ void __launch_bounds__(2 * AdjMainShape<N, EPB>::HALF)
+    adj_main_kernel(const AdjArgs<N> p) {
   constexpr int ND = N * N;
   constexpr int NXY = NS ? 8 : 1;
+  constexpr int NT = AdjMainShape<N, EPB>::NT, HALF = AdjMainShape<N, EPB>::HALF;
+  constexpr int NPART = NS ? 13 : 9;
   __shared__ double ws[EPB][4][ND];
   __shared__ double ps[EPB][5][ND];  // rho, v1, v2, beta, kin
   __shared__ double xys[EPB][NXY][ND];
+  __shared__ double part[NPART][NT];  // the y half's sums
   stage_dependency_sync();  // programmatic dependent launch (see launch_stage_kernel)
-  const int tid = threadIdx.x;
+  const int dir = (int)threadIdx.x / HALF;  // warp-uniform
+  const int tid = (int)threadIdx.x - dir * HALF;
   const int el = tid / ND, node = tid % ND;
   const int e = (int)blockIdx.x * EPB + el;
-  const bool active = e < p.nelem;
+  const bool active = tid < NT && e < p.nelem;
   const int nx = p.cells[0], ny = p.cells[1];
   const int ie = active ? e % nx : 0, je = active ? e / nx : 0;
   double u[4] = {1.0, 0.0, 0.0, 1.0};
   if (active) {
-    double wh[4];
-    load_w_hat<N>(p, ie, je, node, wh);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      ws[el][q][node] = wh[q];
-      u[q] = __ldg(p.u + ((int64_t)e * 4 + q) * ND + node);
+    for (int q = 0; q < 4; ++q) u[q] = __ldg(p.u + ((int64_t)e * 4 + q) * ND + node);
+    if (dir == 0) {
+      double wh[4];
+      load_w_hat<N>(p, ie, je, node, wh);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) ws[el][q][node] = wh[q];
+    } else {
+      const NodeState<2> s = prepare_node<2, VF_CHANDRASHEKAR>(u, p.gamma);
+      ps[el][0][node] = s.rho;
+      ps[el][1][node] = s.v[0];
+      ps[el][2][node] = s.v[1];
+      ps[el][3][node] = s.beta;
+      ps[el][4][node] = s.kin;
     }
-    const NodeState<2> s = prepare_node<2, VF_CHANDRASHEKAR>(u, p.gamma);
-    ps[el][0][node] = s.rho;
-    ps[el][1][node] = s.v[0];
-    ps[el][2][node] = s.v[1];
-    ps[el][3][node] = s.beta;
-    ps[el][4][node] = s.kin;
     if constexpr (NS) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) xys[el][k][node] = __ldg(p.xy + ((int64_t)e * 8 + k) * ND + node);
+      for (int k = 0; k < 4; ++k) {  // rows v * 2 + dir
+        const int r = 2 * k + dir;
+        xys[el][r][node] = __ldg(p.xy + ((int64_t)e * 8 + r) * ND + node);
+      }
     }
   }
   __syncthreads();
-  if (!active) return;
   const int i = node % N, j = node / N;
+  const int pos = dir == 0 ? i : j;
+  const int stride = dir == 0 ? 1 : N, first = dir == 0 ? j * N : i;  // the node's line
   const double lL = p.basis.lhat_l0, lR = p.basis.lhat_rN;
   const double gm1 = p.gamma - 1.0;
-
-  auto node_state = [&](int m) {
-    NodeState<2> s;
-    s.rho = ps[el][0][m];
-    s.v[0] = ps[el][1][m];
-    s.v[1] = ps[el][2][m];
-    s.beta = ps[el][3][m];
-    s.kin = ps[el][4][m];
-    s.p = 0.0;
-    return s;
-  };
-  const NodeState<2> own = node_state(node);
-
-  // -- split-form volume term: every partner on the node's x and y lines
   double rb = 0.0, vb[2] = {0.0, 0.0}, bb = 0.0, kb = 0.0;
-#pragma unroll
-  for (int dir = 0; dir < 2; ++dir) {
-    const int pos = dir == 0 ? i : j;
-    const double n0 = adj_ja<N>(p.tab, dir, 0, ie, je, node);
-    const double n1 = adj_ja<N>(p.tab, dir, 1, ie, je, node);
+  double ub[4] = {0.0, 0.0, 0.0, 0.0};
+  double qb[4] = {0.0, 0.0, 0.0, 0.0};
+  FaceState<2> fo;
+  if (active) {
+    auto node_state = [&](int m) {
+      NodeState<2> s;
+      s.rho = ps[el][0][m];
+      s.v[0] = ps[el][1][m];
+      s.v[1] = ps[el][2][m];
+      s.beta = ps[el][3][m];
+      s.kin = ps[el][4][m];
+      s.p = 0.0;
+      return s;
+    };
+    const NodeState<2> own = node_state(node);
+
+    // -- split-form volume term: every partner on the node's line
+    const double* J0 = p.tab.ja[dir][0] + (int64_t)je * ND;
+    const double* J1 = p.tab.ja[dir][1] + (int64_t)ie * ND;
+    const double n0 = __ldg(J0 + node), n1 = __ldg(J1 + node);
 #pragma unroll
     for (int k = 0; k < N; ++k) {
       if (k == pos) continue;
-      const int mk = dir == 0 ? j * N + k : k * N + i;
-      const double nrm[2] = {0.5 * (n0 + adj_ja<N>(p.tab, dir, 0, ie, je, mk)),
-                             0.5 * (n1 + adj_ja<N>(p.tab, dir, 1, ie, je, mk))};
+      const int mk = first + k * stride;
+      const double nrm[2] = {0.5 * (n0 + __ldg(J0 + mk)), 0.5 * (n1 + __ldg(J1 + mk))};
       const double dik = p.basis.Dsplit[pos][k], dki = p.basis.Dsplit[k][pos];
       double c[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) c[q] = dik * ws[el][q][node] + dki * ws[el][q][mk];
       ec_flux_vjp_left(own, node_state(mk), nrm, c, p.inv_gm1, rb, vb, bb, kb);
     }
-  }
-  double ub[4] = {0.0, 0.0, 0.0, 0.0};
-  const FaceState<2> fo = prepare_face<2>(u, p.gamma);
-  {
-    // beta = rho / (2 p), kin = |v|^2 / 2
-    double ip, iu;
-    two_reciprocals(fo.p, u[0], ip, iu);
-    const double rbt = rb + bb * 0.5 * ip;
-    const double pb = -bb * own.beta * ip;
-    const double vbt[2] = {vb[0] + kb * own.v[0], vb[1] + kb * own.v[1]};
-    prim_to_cons_vjp(u, gm1, rbt, vbt, pb, ub, iu);
-  }
+    fo = prepare_face<2>(u, p.gamma);
 
-  // -- LLF interface fluxes of the element's faces through this node
+    // -- transposed BR1 gradient along the line
+    if constexpr (NS) {
 #pragma unroll
-  for (int dir = 0; dir < 2; ++dir) {
-    const int pos = dir == 0 ? i : j;
+      for (int v = 0; v < 4; ++v) {
+        double s = 0.0;
 #pragma unroll
-    for (int side = 0; side < 2; ++side) {
-      if ((side == 0 && pos != 0) || (side == 1 && pos != N - 1)) continue;
-      const int nie = dir == 0 ? (side ? (ie + 1) % nx : (ie + nx - 1) % nx) : ie;
-      const int nje = dir == 1 ? (side ? (je + 1) % ny : (je + ny - 1) % ny) : je;
+        for (int k = 0; k < N; ++k)
+          s += p.basis.Dhat[k][pos] * xys[el][v * 2 + dir][first + k * stride];
+        qb[v] = s;
+      }
+    }
+
+    // -- the element's face through this node (both faces are never one
+    // node's: n >= 2): LLF interface flux and the BR1 face average
+    if (pos == 0 || pos == N - 1) {
+      const bool hi = pos != 0;
+      const int nie = dir == 0 ? (hi ? (ie + 1) % nx : (ie + nx - 1) % nx) : ie;
+      const int nje = dir == 1 ? (hi ? (je + 1) % ny : (je + ny - 1) % ny) : je;
       const int ne = nie + nx * nje;
-      const int nb_node = dir == 0 ? ((side ? 0 : N - 1) + N * j) : (i + N * (side ? 0 : N - 1));
+      const int nb_node = first + (hi ? 0 : N - 1) * stride;
       double un[4], wn[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) un[q] = __ldg(p.u + ((int64_t)ne * 4 + q) * ND + nb_node);
       load_w_hat<N>(p, nie, nje, nb_node, wn);
       const FaceState<2> fn = prepare_face<2>(un, p.gamma);
       double nrm[2], c[4];
-      if (side == 0) {  // face owned by this element (left state = neighbour)
-        nrm[0] = adj_ja<N>(p.tab, dir, 0, ie, je, node);
-        nrm[1] = adj_ja<N>(p.tab, dir, 1, ie, je, node);
+      // the face belongs to the high-side element (left state = low side)
+      nrm[0] = hi ? adj_ja<N>(p.tab, dir, 0, nie, nje, nb_node) : n0;
+      nrm[1] = hi ? adj_ja<N>(p.tab, dir, 1, nie, nje, nb_node) : n1;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) c[q] = -lL * ws[el][q][node] + lR * wn[q];
-        llf_vjp(fn, fo, nrm, c, false, p.gamma, ub);
-      } else {  // face owned by the high-side neighbour (left state = this node)
-        nrm[0] = adj_ja<N>(p.tab, dir, 0, nie, nje, nb_node);
-        nrm[1] = adj_ja<N>(p.tab, dir, 1, nie, nje, nb_node);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) c[q] = -lL * wn[q] + lR * ws[el][q][node];
-        llf_vjp(fo, fn, nrm, c, true, p.gamma, ub);
+      for (int q = 0; q < 4; ++q) {
+        const double wo = ws[el][q][node];
+        c[q] = hi ? -lL * wn[q] + lR * wo : -lL * wo + lR * wn[q];
       }
-    }
-  }
-
-  // -- transposed BR1 gradient and the direct velocity cotangents
-  if constexpr (NS) {
-    double qb[4];
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      double s = 0.0;
-#pragma unroll
-      for (int k = 0; k < N; ++k) {
-        s += p.basis.Dhat[k][i] * xys[el][v * 2 + 0][j * N + k];
-        s += p.basis.Dhat[k][j] * xys[el][v * 2 + 1][k * N + i];
-      }
-      qb[v] = s;
-    }
-#pragma unroll
-    for (int dir = 0; dir < 2; ++dir) {
-      const int pos = dir == 0 ? i : j;
-#pragma unroll
-      for (int side = 0; side < 2; ++side) {
-        if ((side == 0 && pos != 0) || (side == 1 && pos != N - 1)) continue;
-        const int nie = dir == 0 ? (side ? (ie + 1) % nx : (ie + nx - 1) % nx) : ie;
-        const int nje = dir == 1 ? (side ? (je + 1) % ny : (je + ny - 1) % ny) : je;
-        const int ne = nie + nx * nje;
-        const int nb_node = dir == 0 ? ((side ? 0 : N - 1) + N * j) : (i + N * (side ? 0 : N - 1));
+      FaceState<2> L, R;
+      order_states<2>(hi, fo, fn, L, R);
+      llf_vjp(L, R, nrm, c, hi, p.gamma, ub);
+      if constexpr (NS) {
         // q^ = (q_low + q_high) / 2 lifted into both elements' face nodes
-        const double own_f = side ? lR : -lL;
-        const double nb_f = side ? -lL : lR;
+        const double own_f = hi ? lR : -lL, nb_f = hi ? -lL : lR;
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
           const double xo = xys[el][v * 2 + dir][node];
@@ -456,6 +450,42 @@ __global__ void __launch_bounds__(EPB* N* N) adj_main_kernel(const AdjArgs<N> p)
         }
       }
     }
+    if (dir == 1) {
+      part[0][tid] = rb;
+      part[1][tid] = vb[0];
+      part[2][tid] = vb[1];
+      part[3][tid] = bb;
+      part[4][tid] = kb;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) part[5 + q][tid] = ub[q];
+      if constexpr (NS) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) part[9 + q][tid] = qb[q];
+      }
+    }
+  }
+  __syncthreads();
+  if (!active || dir == 1) return;
+  rb += part[0][tid];
+  vb[0] += part[1][tid];
+  vb[1] += part[2][tid];
+  bb += part[3][tid];
+  kb += part[4][tid];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) ub[q] += part[5 + q][tid];
+  {
+    // beta = rho / (2 p), kin = |v|^2 / 2
+    double ip, iu;
+    two_reciprocals(fo.p, u[0], ip, iu);
+    const double rbt = rb + bb * 0.5 * ip;
+    const double pb = -bb * ps[el][3][node] * ip;
+    const double vbt[2] = {vb[0] + kb * ps[el][1][node], vb[1] + kb * ps[el][2][node]};
+    prim_to_cons_vjp(u, gm1, rbt, vbt, pb, ub, iu);
+  }
+  // -- the direct velocity cotangents of the viscous flux, chain rule
+  if constexpr (NS) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) qb[q] += part[9 + q][tid];
     qb[1] += __ldg(p.qdir + ((int64_t)e * 2 + 0) * ND + node);
     qb[2] += __ldg(p.qdir + ((int64_t)e * 2 + 1) * ND + node);
     // q = (rho, v1, v2, T = p / rho)
