@@ -103,7 +103,7 @@ VARIANT_KERNELS = {
     6: "stage_node2_kernel",
 }
 KERNEL_DESCRIPTIONS = {
-    "stage_line_kernel": "stage_line_kernel (line sweeps, fused RHS + SSPRK3 stage)",
+    "stage_line_kernel": "stage_line_kernel / stage_split_kernel (line sweeps, fused RHS + SSPRK3 stage)",
     "stage_node_kernel": "stage_node_kernel (node-parallel fused RHS + SSPRK3 stage)",
     "stage_pipe_kernel": "stage_pipe_kernel (persistent node-parallel, TMA tile streaming)",
     "stage_node2_kernel": "stage_node2_kernel (node-parallel, two nodes per thread)",

@@ -437,9 +437,9 @@ dgsem_status dgsem_batch_create(const dgsem_mesh_desc* meshes, int n_meshes,
     for (int f = 0; f < 6; ++f) c.bc.kind[f] = 0;
     g.members = kv.second;
     // tile arrays sized for one element per tile (any launch shape fits)
-    g.engine->set_variant(0);
     size_t max_tiles = 0;
     for (int m : g.members) max_tiles += (size_t)b->nelem[m];
+    g.engine->set_mesh_size((int64_t)max_tiles);
     g.tile_capacity = max_tiles;
     g.tile_mesh = balloc<int>(b, max_tiles);
     g.tile_e0 = balloc<int>(b, max_tiles);

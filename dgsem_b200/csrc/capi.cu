@@ -330,6 +330,7 @@ dgsem_status dgsem_ctx_create(const dgsem_mesh_desc* mesh,
     conserved_from_primitive(pre, scheme->gamma, c.bc.dmr_pre);
     c.bc.sqrt3 = std::sqrt(3.0);
   }
+  ctx->engine->set_mesh_size(c.nelem);
   ctx->nodes = nd == 2 ? n * n : n * n * n;
   ctx->nvars = nd + 2;
   ctx->state_len = c.nelem * ctx->nodes * ctx->nvars;

@@ -49,7 +49,7 @@ struct EngineConfig {
   int skip_tile_copy;
 };
 
-// Launch-shape variants: 0-2 line sweeps (stage_line_kernel.cuh), 3-4
+// Launch-shape variants: 0-2 line shapes (stage_line_kernel.cuh), 3-4
 // node-parallel (stage_node_kernel.cuh), 5 persistent node-parallel with TMA
 // tile streaming (stage_pipe_kernel.cuh; single-mesh launches; split form
 // without shock capturing or viscous terms, an even number of doubles per
@@ -89,6 +89,9 @@ class EngineBase {
   // launch-shape variant in [0, num_variants())
   virtual void set_variant(int v) = 0;
   virtual int variant() const = 0;
+  // elements of the mesh (of all meshes of a batch group): launch shape 0
+  // depends on it
+  virtual void set_mesh_size(int64_t nelem) = 0;
   virtual int num_variants() const = 0;
 };
 
@@ -141,13 +144,22 @@ inline StageArgs<N> stage_args_common(const EngineConfig& cfg, double a, double 
   return args;
 }
 
-// Line-sweep variants 0-2 (stage_line_kernel): warps per block and resident
-// blocks per SM requested from the register allocator.
-template <int N, int V>
+// Line shapes (stage_line_kernel.cuh): 0 = the split or the sweep form by the
+// mesh's size (Engine::split_by_size), 1 = split, 2 = sweep with another
+// register cap than 0's.  Resident blocks per SM requested from the register
+// allocator: the sweeps get 168 registers (12 warps per SM) where a line's
+// data fit them, 255 (8 warps) at long lines, and shape 2 128 (16 warps) at
+// short ones (2D n = 2: 111 us per stage of 640 000 elements against 116).
+template <int DIM, int N, int V>
 struct LineLaunch {
-  static constexpr int WPB = V == 2 ? 4 : 2;
-  static constexpr int MINB = V == 0 ? 6 : V == 1 ? 8 : N > 4 ? 2 : 3;
+  static constexpr int WPB = 2;
+  static constexpr bool LONG = N > 5 || (DIM == 3 && N == 5);
+  static constexpr int MINB = V == 0 ? (LONG ? 4 : 6) : N <= 4 ? 8 : LONG ? 6 : 4;
   static constexpr int NT = 32 * WPB;
+};
+template <int DIM, int N, bool HG>
+struct SplitLaunch {
+  static constexpr int MINB = DIM == 3 ? 2 : N <= 4 ? (HG ? 3 : 4) : N <= 6 ? (HG ? 2 : 3) : 2;
 };
 
 // Fraction of the lanes of its warps that a block of `threads` threads uses.
@@ -233,26 +245,81 @@ class Engine final : public EngineBase {
  public:
   static constexpr bool kBatch = !NS && !HG;
 
+  using LG = LineGeo<DIM, N>;
+  using SSh = SplitShape<DIM, N, VF, HG>;
   template <int V, bool B>
   static auto line_kernel() {
-    return stage_line_kernel<DIM, N, VF, SF, HG, NS, B, LineLaunch<N, V>::WPB, LineLaunch<N, V>::MINB>;
+    using L = LineLaunch<DIM, N, V>;
+    return stage_line_kernel<DIM, N, VF, SF, HG, NS, B, L::WPB, L::MINB>;
   }
-  template <int V>
-  static constexpr size_t line_smem() {
-    return LineShape<DIM, N, VF>::smem_bytes(LineLaunch<N, V>::WPB);
+  template <bool B>
+  static auto split_kernel() {
+    return stage_split_kernel<DIM, N, VF, SF, HG, NS, B, SplitLaunch<DIM, N, HG>::MINB>;
   }
-  template <int V>
-  static constexpr int line_epb() {
-    return LineGeo<DIM, N>::EPW * LineLaunch<N, V>::WPB;
+  static constexpr int LINE_WPB = LineLaunch<DIM, N, 0>::WPB;
+  static constexpr int LINE_NT = LineLaunch<DIM, N, 0>::NT;
+  static constexpr int LINE_EPB = LG::EPW * LINE_WPB;
+  static constexpr size_t LINE_SMEM = LineShape<DIM, N, VF>::smem_bytes(LINE_WPB);
+  // whether the current line shape runs in the split form
+  bool use_split() const { return variant_ == 1 || (variant_ == 0 && split_); }
+
+  // Loads and configures the kernels of one launch shape (and of its batched
+  // and fallback forms), once per engine: only shapes that are selected, since
+  // a kernel's code goes to the device at its first use.
+  void load_variant(int v) {
+    if (loaded_ & (1u << v)) return;
+    loaded_ |= 1u << v;
+    auto attr = [](auto kernel, size_t smem) {
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    };
+    auto node = [&](auto cap) {
+      constexpr bool CAP = decltype(cap)::value;
+      attr(node_kernel<false, CAP>(), NSh::smem_bytes);
+      if constexpr (kBatch) attr(node_kernel<true, CAP>(), NSh::smem_bytes);
+    };
+    auto sweep = [&](auto v_c) {
+      constexpr int V = decltype(v_c)::value;
+      attr(line_kernel<V, false>(), LINE_SMEM);
+      if constexpr (kBatch) attr(line_kernel<V, true>(), LINE_SMEM);
+    };
+    if constexpr (NS) set_viscous_flux_attributes<DIM, N>();
+    if (v == 1 || (v == 0 && split_)) {
+      attr(split_kernel<false>(), SSh::smem_bytes);
+      if constexpr (kBatch) attr(split_kernel<true>(), SSh::smem_bytes);
+    } else if (v == 0) {
+      sweep(std::integral_constant<int, 0>{});
+    } else if (v == 2) {
+      sweep(std::integral_constant<int, 2>{});
+    } else if (v == 4) {
+      node(std::false_type{});
+    } else {
+      node(std::true_type{});  // 3; 5 and 6 fall back to it
+    }
+    if constexpr (kPipe)
+      if (v == 5) attr(pipe_kernel(), PSh::smem_bytes);
+    if constexpr (kNode2)
+      if (v == 6) attr(node2_kernel(), Node2Shape<N, VF>::smem_bytes);
   }
 
-  template <int V>
-  static void set_attributes() {
-    cudaFuncSetAttribute(line_kernel<V, false>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)line_smem<V>());
-    if constexpr (kBatch)
-      cudaFuncSetAttribute(line_kernel<V, true>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)line_smem<V>());
+  // Shape 0 runs the split form on meshes too small to fill the GPU with one
+  // warp per group of elements (`warps` of the sweep); both give the same
+  // bits.  us per stage on a B200, split / sweep, near the crossings:
+  //   2D n = 3   723 warps 5.7 / 7.1, 2 161: 11.0 / 10.1
+  //      n = 4  1513: 10.8 / 12.2, 3 200: 18.7 / 15.5 (64^2 elements 4.7 / 6.3)
+  //      n = 6  2290: 27.0 / 27.6, 14 259: 173 / 107
+  //      n = 8  1600: 35 / 50, 10 000: 191 / 124
+  //      shock capturing n = 4: 32: 7.1 / 13, 1 800: 21.4 / 24.8, 3 200: 25.6 /
+  //      18.1; n = 5: 960: 31 / 28, 2 731: 37 / 26
+  //   3D n = 4   108: 2.9 / 6.9, 1 372: 13.5 / 10.1
+  //      n = 5   125: 3.2 / 9.3, 1 331: 14.4 / 14.2
+  void set_mesh_size(int64_t nelem) override {
+    const int64_t warps = (nelem + LG::EPW - 1) / LG::EPW;
+    split_ = warps < split_below();
+    loaded_ &= ~1u;
+    load_variant(variant_);
+  }
+  static constexpr int64_t split_below() {
+    return DIM == 3 ? 700 : HG ? (N > 4 ? 800 : 2000) : N <= 3 ? 1400 : 2400;
   }
 
   // node-parallel shapes: split form with shock capturing or with the
@@ -339,29 +406,6 @@ class Engine final : public EngineBase {
     }
   }
 
-  Engine() {
-    set_attributes<0>();
-    set_attributes<1>();
-    set_attributes<2>();
-    if constexpr (NS) set_viscous_flux_attributes<DIM, N>();
-    if constexpr (kNode) {
-      const int sm = (int)NSh::smem_bytes;
-      cudaFuncSetAttribute(node_kernel<false, true>(), cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-      cudaFuncSetAttribute(node_kernel<false, false>(), cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    }
-    if constexpr (kBatch) {
-      const int sm = (int)NSh::smem_bytes;
-      cudaFuncSetAttribute(node_kernel<true, true>(), cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-      cudaFuncSetAttribute(node_kernel<true, false>(), cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    }
-    if constexpr (kPipe)
-      cudaFuncSetAttribute(pipe_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)PSh::smem_bytes);
-    if constexpr (kNode2)
-      cudaFuncSetAttribute(node2_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)Node2Shape<N, VF>::smem_bytes);
-  }
-
   StageArgs<N> common_args(const EngineConfig& cfg, double a, double b, double t,
                            const double* t_dev, double* alpha_out) const {
     StageArgs<N> args = stage_args_common<N>(cfg, a, b, t, t_dev, alpha_out);
@@ -371,12 +415,15 @@ class Engine final : public EngineBase {
     return args;
   }
 
-  template <int V>
-  void launch(const StageArgs<N>& args, int64_t nelem, cudaStream_t s) const {
-    const int64_t blocks = (nelem + line_epb<V>() - 1) / line_epb<V>();
-    last_grid_ = blocks;
-    launch_stage_kernel(line_kernel<V, false>(), (unsigned)blocks, LineLaunch<N, V>::NT,
-                        line_smem<V>(), s, args);
+  // line shapes; `grid` blocks of elements_per_block() elements
+  template <bool B>
+  void launch_line(const StageArgs<N>& args, unsigned grid, cudaStream_t s) const {
+    if (use_split())
+      launch_stage_kernel(split_kernel<B>(), grid, SSh::NT, SSh::smem_bytes, s, args);
+    else if (variant_ == 2)
+      launch_stage_kernel(line_kernel<2, B>(), grid, LINE_NT, LINE_SMEM, s, args);
+    else
+      launch_stage_kernel(line_kernel<0, B>(), grid, LINE_NT, LINE_SMEM, s, args);
   }
 
   cudaError_t stage(const EngineConfig& cfg, const double* u_n,
@@ -399,24 +446,18 @@ class Engine final : public EngineBase {
     args.mesh.mij = cfg.mij;
     if constexpr (NS) launch_viscous_flux<DIM, N>(cfg, u_in, cfg.visc, cfg.grad, s);
     switch (variant_) {
-      case 1: launch<1>(args, cfg.nelem, s); break;
-      case 2: launch<2>(args, cfg.nelem, s); break;
       case 3: launch_node<true>(args, cfg.nelem, s); break;
       case 4: launch_node<false>(args, cfg.nelem, s); break;
       case 5: launch_pipe(args, cfg.nelem, s); break;
       case 6: launch_node2(args, cfg.nelem, s); break;
-      default: launch<0>(args, cfg.nelem, s); break;
+      default: {
+        last_grid_ = (cfg.nelem + elements_per_block() - 1) / elements_per_block();
+        launch_line<false>(args, (unsigned)last_grid_, s);
+        break;
+      }
     }
     if (diag) last_diag_slots_ = last_grid_;
     return cudaGetLastError();
-  }
-
-  template <int V>
-  void launch_batch(const StageArgs<N>& args, int ntiles, cudaStream_t s) const {
-    if constexpr (kBatch) {
-      launch_stage_kernel(line_kernel<V, true>(), (unsigned)ntiles, LineLaunch<N, V>::NT,
-                          line_smem<V>(), s, args);
-    }
   }
 
   cudaError_t batch_stage(const EngineConfig& cfg, const MeshView* meshes,
@@ -431,13 +472,11 @@ class Engine final : public EngineBase {
       args.tile_mesh = tile_mesh;
       args.tile_e0 = tile_e0;
       switch (variant_) {
-        case 1: launch_batch<1>(args, ntiles, s); break;
-        case 2: launch_batch<2>(args, ntiles, s); break;
         case 3:
         case 5:
         case 6: launch_node_batch<true>(args, ntiles, s); break;
         case 4: launch_node_batch<false>(args, ntiles, s); break;
-        default: launch_batch<0>(args, ntiles, s); break;
+        default: launch_line<true>(args, (unsigned)ntiles, s); break;
       }
       return cudaGetLastError();
     }
@@ -457,27 +496,30 @@ class Engine final : public EngineBase {
     if constexpr (kNode2)
       if (variant_ == 6) return Node2Launch<N>::EPB;
     if (variant_ >= 3) return NL::EPB;
-    return variant_ == 2 ? line_epb<2>() : variant_ == 1 ? line_epb<1>() : line_epb<0>();
+    return use_split() ? LG::EPW : LINE_EPB;
   }
   int threads_per_block() const override {
     if (variant_ >= 3) return NL::NT;
-    return variant_ == 2 ? LineLaunch<N, 2>::NT
-           : variant_ == 1 ? LineLaunch<N, 1>::NT
-                           : LineLaunch<N, 0>::NT;
+    return use_split() ? SSh::NT : LINE_NT;
   }
   size_t smem_bytes() const override {
     if constexpr (kNode2)
       if (variant_ == 6) return Node2Shape<N, VF>::smem_bytes;
     if (variant_ >= 3) return NSh::smem_bytes;
-    return variant_ == 2 ? line_smem<2>() : variant_ == 1 ? line_smem<1>() : line_smem<0>();
+    return use_split() ? SSh::smem_bytes : LINE_SMEM;
   }
-  void set_variant(int v) override { variant_ = (v >= 0 && v < num_variants()) ? v : 0; }
+  void set_variant(int v) override {
+    variant_ = (v >= 0 && v < num_variants()) ? v : 0;
+    load_variant(variant_);
+  }
   int variant() const override { return variant_; }
   // shapes 5 and 6 exist for single-mesh launches; batched launches run them as 3
   int num_variants() const override { return kNode2 ? 7 : kPipe ? 6 : kNode ? 5 : 3; }
 
  private:
   int variant_ = 0;
+  bool split_ = false;   // shape 0 runs the split form (set_mesh_size)
+  unsigned loaded_ = 0;  // launch shapes configured so far (load_variant)
   mutable int64_t pipe_blocks_ = 0;
   mutable int64_t last_grid_ = 0;  // blocks of the last single-mesh stage launch
   int64_t last_diag_slots_ = 0;

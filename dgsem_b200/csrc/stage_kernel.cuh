@@ -274,11 +274,11 @@ __device__ __forceinline__ void reflect_state(const double* ui, const double* n,
   const double rho = ui[0];
   const double vx = ui[1] / rho;
   const double vy = ui[2] / rho;
-  const double nn2 = n[0] * n[0] + n[1] * n[1];
-  const double vn = (vx * n[0] + vy * n[1]) / nn2;
+  const double nn2 = __fma_rn(n[1], n[1], __dmul_rn(n[0], n[0]));
+  const double vn = __fma_rn(vy, n[1], __dmul_rn(vx, n[0])) / nn2;
   uw[0] = rho;
-  uw[1] = rho * (vx - 2.0 * vn * n[0]);
-  uw[2] = rho * (vy - 2.0 * vn * n[1]);
+  uw[1] = __dmul_rn(rho, __fma_rn(-2.0 * vn, n[0], vx));
+  uw[2] = __dmul_rn(rho, __fma_rn(-2.0 * vn, n[1], vy));
   uw[3] = ui[3];
 }
 

@@ -28,8 +28,7 @@
 //   * the volume term is one straight block without branches: reciprocals and
 //     roots are branch-free (physics.cuh: recip, root) and the logarithmic
 //     means take their series for every pair; a line with a pair outside the
-//     series' range repeats its volume term in a small general loop
-//     (line_volume_general).
+//     series' range repeats its volume term (LineMean).
 //
 // Shared memory of a warp, planes of doubles [slot][element][node]: the NV
 // conserved variables, 1 / (2 rho), p, Chandrashekar: rho / p; then the NV
@@ -229,15 +228,34 @@ struct LineScale {
   static constexpr double value = VF == VF_KENNEDY_GRUBER ? 0.25 : 0.5;
 };
 
-// Two-point volume flux of two nodes of a line, ns = Ja_i + Ja_k.  GENERAL:
-// the logarithmic means with the reference's branch rule; otherwise their
-// series alone, and *outside is set when a pair is not in the series' range
-// (the flux is then not to be used).  The series of the mean multiplies its
-// f^2 = ((a-b)/(a+b))^2 < 1e-4 by coefficients of order one, so the reciprocal
-// of a + b in f needs 12 digits only; the inverse mean's is full precision.
-template <int DIM, int VF, bool GENERAL>
+// How a line evaluates the logarithmic means of its pairs, from f^2 =
+// ((a - b) / (a + b))^2 of both means:
+//   MEAN_SHORT    f^2 < 1e-4: the reference's series (4 terms); the series of
+//                 the mean multiplies f^2 by coefficients of order one, so the
+//                 reciprocal of a + b in f needs 12 digits only
+//   MEAN_LONG     f^2 < 1/16 (a ratio of up to 5/3 between two nodes): the
+//                 same series atanh(f) / f = sum f^2k / (2k + 1) to 13 terms
+//                 (remainder below 1e-17).  The reference takes the logarithm
+//                 here, whose argument b / a near 1 costs it up to 50 units in
+//                 the last place; the two agree to that
+//   MEAN_GENERAL  any pair: the reference's rule with the logarithm
+// A line takes the same form for all of its pairs, so each form is one block
+// of straight code.
+enum LineMean : int { MEAN_SHORT, MEAN_LONG, MEAN_GENERAL };
+
+__device__ __forceinline__ double line_atanh_series(double t) {
+  double r = 1.0 / 25.0;
+#pragma unroll
+  for (int k = 11; k >= 0; --k) r = __fma_rn(r, t, 1.0 / (2 * k + 1));
+  return r;
+}
+
+// Two-point volume flux of two nodes of a line, ns = Ja_i + Ja_k.  *range
+// keeps the largest high word of the f^2 seen (MEAN_SHORT; the caller compares
+// it with the range of the form).
+template <int DIM, int VF, int MEAN>
 __device__ __forceinline__ void line_pair_flux(const LineNode<DIM>& L, const LineNode<DIM>& R,
-                                               const double* ns, double inv_gm1, bool* outside,
+                                               const double* ns, double inv_gm1, int* range,
                                                double* f) {
   const double rs = L.rho + R.rho;
   double va[DIM];
@@ -266,13 +284,19 @@ __device__ __forceinline__ void line_pair_flux(const LineNode<DIM>& L, const Lin
   const double s = a + b;
   const double is = recip(s);
   double rho_mean, im;
-  if constexpr (GENERAL) {
+  if constexpr (MEAN == MEAN_GENERAL) {
     rho_mean = ln_mean_rs(L.rho, R.rho, rs, recip(rs));
     im = inv_ln_mean_rs(a, b, is);
+  } else if constexpr (MEAN == MEAN_LONG) {
+    const double t = (L.rho - R.rho) * recip(rs), g2 = __dmul_rn(t, t);
+    const double w = (a - b) * is, f2 = __dmul_rn(w, w);
+    rho_mean = __dmul_rn(0.5 * rs, recip(line_atanh_series(g2)));
+    im = __dmul_rn(2.0 * is, line_atanh_series(f2));
   } else {
     const double t = (L.rho - R.rho) * recip_approx(rs), g2 = __dmul_rn(t, t);
     const double w = (a - b) * is, f2 = __dmul_rn(w, w);
-    *outside |= !(fmax(g2, f2) < 1.0e-4);
+    // both are >= 0 or NaN: compared on the high words, no FP64 compare
+    *range = max(*range, max(__double2hiint(g2), __double2hiint(f2)));
     rho_mean = __dmul_rn(
         rs, __fma_rn(g2, __fma_rn(g2, __fma_rn(g2, -22.0 / 945.0, -2.0 / 45.0), -1.0 / 6.0), 0.5));
     im = __dmul_rn(
@@ -419,68 +443,13 @@ __device__ __forceinline__ LineNode<DIM> line_node_data(const double* P, int o) 
   return q;
 }
 
-// Volume term of one line with the general two-point flux, pair by pair,
-// added to R with the factor `scale`.  Rolled up: it runs for the few lines
-// with a jump of more than about 2 % between two nodes.
-template <int DIM, int N, int VF>
-__device__ __forceinline__ void line_volume_general(const StageArgs<N>& p, const MeshView& M,
-                                                    const LineElement<DIM>& E, int dir,
-                                                    const LinePos<DIM, N>& pos, const double* P,
-                                                    double* R, double scale) {
-  using G = LineGeo<DIM, N>;
-  auto slot = [&](int m) {
-    int o = pos.off[0];
-#pragma unroll
-    for (int k = 1; k < N; ++k) o = m == k ? pos.off[k] : o;
-    return o;
-  };
-#pragma unroll 1
-  for (int i = 0; i + 1 < N; ++i) {
-    const int oi = slot(i);
-    const LineNode<DIM> L = line_node_data<DIM, VF, G::PLANE>(P, oi);
-#pragma unroll 1
-    for (int k = i + 1; k < N; ++k) {
-      const int ok = slot(k);
-      const LineNode<DIM> Q = line_node_data<DIM, VF, G::PLANE>(P, ok);
-      double ns[DIM], f[G::NV];
-#pragma unroll
-      for (int c = 0; c < DIM; ++c) {
-        const double* J = M.tab.ja[dir][c] + (int64_t)E.row[c] * G::ND + pos.first;
-        ns[c] = __ldg(J + i * pos.stride) + __ldg(J + k * pos.stride);
-      }
-      line_pair_flux<DIM, VF, true>(L, Q, ns, p.inv_gm1, nullptr, f);
-      const double dik = scale * p.basis.Dvol[i][k], dki = scale * p.basis.Dvol[k][i];
-#pragma unroll
-      for (int v = 0; v < G::NV; ++v) {
-        R[v * G::PLANE + oi] = __fma_rn(dik, f[v], R[v * G::PLANE + oi]);
-        R[v * G::PLANE + ok] = __fma_rn(dki, f[v], R[v * G::PLANE + ok]);
-      }
-    }
-  }
-}
-
-// One direction of a lane's line; its contribution is added to R (FIRST:
-// written), and left in acc for the last direction at odd n.
-template <int DIM, int N, int VF, int SF, bool HG, bool NS, bool XL>
-__device__ __forceinline__ void line_sweep(const StageArgs<N>& p, const MeshView& M,
-                                           const LineElement<DIM>& E, int dir, int el, int line,
-                                           const double* P, double* R, double alpha,
-                                           double t_stage, double (*acc)[DIM + 2],
-                                           LinePos<DIM, N>& pos) {
-  using G = LineGeo<DIM, N>;
-  using K = LineSlots<DIM, VF>;
-  constexpr int NV = G::NV, ND = G::ND, NF = G::NF, PLANE = G::PLANE;
-  const double gamma = p.gamma;
-  pos.set(dir, el, line);
-  // global loads of the direction: neighbours' traces, metric terms of the
-  // line, and the normal of the high face
-  int nb[2];
-  nb[0] = __ldg(E.info + 6 + 2 * dir);
-  nb[1] = __ldg(E.info + 7 + 2 * dir);
-  double ja[N][DIM], nh[DIM];
+// Metric terms of a line.
+template <int DIM, int N, bool XL>
+__device__ __forceinline__ void line_metrics(const MeshView& M, const LineElement<DIM>& E, int dir,
+                                             const LinePos<DIM, N>& pos, double (*ja)[DIM]) {
 #pragma unroll
   for (int c = 0; c < DIM; ++c) {
-    const double* J = M.tab.ja[dir][c] + (int64_t)E.row[c] * ND + pos.first;
+    const double* J = M.tab.ja[dir][c] + (int64_t)E.row[c] * LineGeo<DIM, N>::ND + pos.first;
     if constexpr (XL) {
       double v[N];
       load_xline<N, true>(J, v);
@@ -491,7 +460,37 @@ __device__ __forceinline__ void line_sweep(const StageArgs<N>& p, const MeshView
       for (int m = 0; m < N; ++m) ja[m][c] = __ldg(J + m * pos.stride);
     }
   }
-  double tr[2][NV];
+}
+
+// The neighbours across a line's ends and the normal of its high face: Ja^dir
+// of the element on the high side at its low face (at a boundary the line's
+// own last node).  The component along dir does not depend on the position
+// along dir.
+template <int DIM, int N>
+__device__ __forceinline__ void line_ends(const MeshView& M, const LineElement<DIM>& E, int dir,
+                                          const LinePos<DIM, N>& pos, int* nb, double* nh) {
+  constexpr int ND = LineGeo<DIM, N>::ND;
+  nb[0] = __ldg(E.info + 6 + 2 * dir);
+  nb[1] = __ldg(E.info + 7 + 2 * dir);
+  const int cd = M.cells[dir];
+  const int step = nb[1] > E.e ? 1 : 1 - cd;  // the neighbour's position along dir
+#pragma unroll
+  for (int c = 0; c < DIM; ++c) {
+    // stride of dir in the rows of axis c
+    const int st = DIM == 2 ? 1
+                   : c == 0 ? (dir == 1 ? 1 : M.cells[1])
+                            : (dir == 0 ? 1 : M.cells[0]);
+    const int shift = c == dir || nb[1] < 0 ? 0 : step * st;
+    nh[c] = __ldg(M.tab.ja[dir][c] + (int64_t)(E.row[c] + shift) * ND + pos.first +
+                  (nb[1] < 0 ? (N - 1) * pos.stride : 0));
+  }
+}
+
+// The neighbours' conserved states at a line's ends.
+template <int DIM, int N>
+__device__ __forceinline__ void line_traces(const MeshView& M, const LinePos<DIM, N>& pos,
+                                            const int* nb, double (*tr)[DIM + 2]) {
+  constexpr int NV = DIM + 2, ND = LineGeo<DIM, N>::ND;
 #pragma unroll
   for (int s = 0; s < 2; ++s) {
     const double* T = M.u_in + (int64_t)max(nb[s], 0) * (NV * ND) + pos.first +
@@ -499,71 +498,18 @@ __device__ __forceinline__ void line_sweep(const StageArgs<N>& p, const MeshView
 #pragma unroll
     for (int v = 0; v < NV; ++v) tr[s][v] = __ldg(T + v * ND);
   }
-  // The face normal is Ja^dir of the element on the high side at its low
-  // face.  Its component along dir does not depend on the position along dir.
-  {
-    const int cd = M.cells[dir];
-    const int step = nb[1] > E.e ? 1 : 1 - cd;  // the neighbour's position along dir
-#pragma unroll
-    for (int c = 0; c < DIM; ++c) {
-      // stride of dir in the rows of axis c
-      const int st = DIM == 2 ? 1
-                     : c == 0 ? (dir == 1 ? 1 : M.cells[1])
-                              : (dir == 0 ? 1 : M.cells[0]);
-      const int shift = c == dir || nb[1] < 0 ? 0 : step * st;
-      nh[c] = __ldg(M.tab.ja[dir][c] + (int64_t)(E.row[c] + shift) * ND + pos.first +
-                    (nb[1] < 0 ? (N - 1) * pos.stride : 0));
-    }
-  }
+}
 
-  // the line's nodes
-  LineNode<DIM> q[N];
-  double end[2][NV], ehinv[2];
-  {
-    double hinv[N], t[N];
-    load_line<XL, N>(P + K::HINV * PLANE, pos.off, hinv);
-    ehinv[0] = hinv[0];
-    ehinv[1] = hinv[N - 1];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      if (v == NV - 1 && VF != VF_KENNEDY_GRUBER) {
-        t[0] = P[v * PLANE + pos.off[0]];
-        t[N - 1] = P[v * PLANE + pos.off[N - 1]];
-      } else {
-        load_line<XL, N>(P + v * PLANE, pos.off, t);
-      }
-      end[0][v] = t[0];
-      end[1][v] = t[N - 1];
-      if (v == 0) {
-#pragma unroll
-        for (int m = 0; m < N; ++m) q[m].rho = t[m];
-      } else if (v <= DIM) {
-#pragma unroll
-        for (int m = 0; m < N; ++m) q[m].hv[v - 1] = __dmul_rn(t[m], hinv[m]);
-      } else if (VF == VF_KENNEDY_GRUBER) {
-#pragma unroll
-        for (int m = 0; m < N; ++m) q[m].x = __dmul_rn(t[m], hinv[m]);
-      }
-    }
-    load_line<XL, N>(P + K::P * PLANE, pos.off, t);
-#pragma unroll
-    for (int m = 0; m < N; ++m) q[m].p = t[m];
-    if constexpr (VF == VF_CHANDRASHEKAR) {
-      load_line<XL, N>(P + K::B * PLANE, pos.off, t);
-#pragma unroll
-      for (int m = 0; m < N; ++m) {
-        q[m].x = t[m];
-        q[m].y = line_dot<DIM>(q[m].hv, q[m].hv);
-      }
-    }
-  }
-
-  // volume term: every pair of the line once
+// Every pair of the line once, with one form of the means.
+template <int DIM, int N, int VF, int MEAN>
+__device__ __forceinline__ int line_pairs(const StageArgs<N>& p, const LineNode<DIM>* q,
+                                          const double (*ja)[DIM], double (*acc)[DIM + 2]) {
+  constexpr int NV = DIM + 2;
 #pragma unroll
   for (int m = 0; m < N; ++m)
 #pragma unroll
     for (int v = 0; v < NV; ++v) acc[m][v] = 0.0;
-  bool outside = false;
+  int range = 0;
 #pragma unroll
   for (int i = 0; i < N; ++i)
 #pragma unroll
@@ -572,7 +518,7 @@ __device__ __forceinline__ void line_sweep(const StageArgs<N>& p, const MeshView
       double ns[DIM], f[NV];
 #pragma unroll
       for (int c = 0; c < DIM; ++c) ns[c] = ja[i][c] + ja[k][c];
-      line_pair_flux<DIM, VF, false>(q[i], q[k], ns, p.inv_gm1, &outside, f);
+      line_pair_flux<DIM, VF, MEAN>(q[i], q[k], ns, p.inv_gm1, &range, f);
       const double dik = p.basis.Dvol[i][k], dki = p.basis.Dvol[k][i];
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
@@ -580,61 +526,182 @@ __device__ __forceinline__ void line_sweep(const StageArgs<N>& p, const MeshView
         acc[k][v] = __fma_rn(dki, f[v], acc[k][v]);
       }
     }
-  const bool troubled = HG && fabs(alpha - 0.0) > p.atol;
-  if (VF != VF_KENNEDY_GRUBER && outside) {
-    if (dir == 0) {
+  return range;
+}
+
+// Node data of a line.
+template <int DIM, int N, int VF, bool XL>
+__device__ __forceinline__ void line_nodes(const double* P, const LinePos<DIM, N>& pos,
+                                           LineNode<DIM>* q) {
+  using K = LineSlots<DIM, VF>;
+  constexpr int NV = DIM + 2, PLANE = LineGeo<DIM, N>::PLANE;
+  double hinv[N], t[N];
+  load_line<XL, N>(P + K::HINV * PLANE, pos.off, hinv);
 #pragma unroll
-      for (int v = 0; v < NV; ++v)
+  for (int v = 0; v < NV; ++v) {
+    if (v == NV - 1 && VF != VF_KENNEDY_GRUBER) continue;
+    load_line<XL, N>(P + v * PLANE, pos.off, t);
+    if (v == 0) {
 #pragma unroll
-        for (int m = 0; m < N; ++m) R[v * PLANE + pos.off[m]] = 0.0;
+      for (int m = 0; m < N; ++m) q[m].rho = t[m];
+    } else if (v <= DIM) {
+#pragma unroll
+      for (int m = 0; m < N; ++m) q[m].hv[v - 1] = __dmul_rn(t[m], hinv[m]);
+    } else if (VF == VF_KENNEDY_GRUBER) {
+#pragma unroll
+      for (int m = 0; m < N; ++m) q[m].x = __dmul_rn(t[m], hinv[m]);
     }
-    line_volume_general<DIM, N, VF>(p, M, E, dir, pos, P, R, troubled ? 1.0 - alpha : 1.0);
-#pragma unroll
-    for (int m = 0; m < N; ++m)
-#pragma unroll
-      for (int v = 0; v < NV; ++v) acc[m][v] = 0.0;
   }
-  if constexpr (HG) {
-    if (troubled) {
-      // volume_flux.hpp:817-842: (1 - alpha) DG + alpha FV, the FV subcell
-      // fluxes (:457-509 in 2D, :521-630 in 3D) once per interface
-      const double one_m = 1.0 - alpha;
+  load_line<XL, N>(P + K::P * PLANE, pos.off, t);
 #pragma unroll
-      for (int m = 0; m < N; ++m)
+  for (int m = 0; m < N; ++m) q[m].p = t[m];
+  if constexpr (VF == VF_CHANDRASHEKAR) {
+    load_line<XL, N>(P + K::B * PLANE, pos.off, t);
 #pragma unroll
-        for (int v = 0; v < NV; ++v) acc[m][v] = __dmul_rn(acc[m][v], one_m);
-      auto node = [&](int m) {
-        LineFace<DIM> s;
+    for (int m = 0; m < N; ++m) {
+      q[m].x = t[m];
+      q[m].y = line_dot<DIM>(q[m].hv, q[m].hv);
+    }
+  }
+}
+
+// Adds `scale` times the volume term of a line outside the short series' range
+// to its line of R: with the long series, or (not `series`) the general means,
+// the latter rolled up for n > 4.  A function of its own, called by few lines
+// and last, when little is live: inlined, its code cost the kernels' main path
+// registers (TGV 32^3 Chandrashekar 96 -> 111 us per stage, KH 1024^2 445 ->
+// 471).
+template <int DIM, int N, int VF>
+__device__ __noinline__ void line_volume_steep(const StageArgs<N>* p, const MeshView* M,
+                                               LineElement<DIM> E, int dir, int el, int line,
+                                               const double* P, double* R, bool series,
+                                               double scale) {
+  using G = LineGeo<DIM, N>;
+  constexpr int NV = G::NV, PLANE = G::PLANE;
+  LinePos<DIM, N> pos;
+  pos.set(dir, el, line);
+  LineNode<DIM> q[N];
+  double ja[N][DIM], acc[N][NV];
+  if (series || N <= 4) {
+    line_nodes<DIM, N, VF, false>(P, pos, q);
+    line_metrics<DIM, N, false>(*M, E, dir, pos, ja);
+    if (series)
+      line_pairs<DIM, N, VF, MEAN_LONG>(*p, q, ja, acc);
+    else if constexpr (N <= 4)
+      line_pairs<DIM, N, VF, MEAN_GENERAL>(*p, q, ja, acc);
 #pragma unroll
-        for (int v = 0; v < NV; ++v) s.u[v] = P[v * PLANE + pos.off[m]];
+    for (int v = 0; v < NV; ++v)
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) s.hv[d] = q[m].hv[d];
-        s.p = q[m].p;
-        s.qa2 = __dmul_rn(__dmul_rn(0.5 * gamma, s.p), P[K::HINV * PLANE + pos.off[m]]);
-        return s;
-      };
-      LineFace<DIM> L = node(0);
+      for (int m = 0; m < N; ++m) {
+        double* r = R + v * PLANE + pos.off[m];
+        *r = __fma_rn(scale, acc[m][v], *r);
+      }
+    return;
+  }
+#pragma unroll 1
+  for (int i = 0; i + 1 < N; ++i) {
+    const int oi = LinePos<DIM, N>::slot(dir, el, line, i);
+    const LineNode<DIM> L = line_node_data<DIM, VF, PLANE>(P, oi);
+#pragma unroll 1
+    for (int k = i + 1; k < N; ++k) {
+      const int ok = LinePos<DIM, N>::slot(dir, el, line, k);
+      const LineNode<DIM> Q = line_node_data<DIM, VF, PLANE>(P, ok);
+      double ns[DIM], f[NV];
 #pragma unroll
-      for (int m = 1; m < N; ++m) {
-        const LineFace<DIM> S = node(m);
-        double nrm[DIM], f[NV];
+      for (int c = 0; c < DIM; ++c) {
+        const double* J = M->tab.ja[dir][c] + (int64_t)E.row[c] * G::ND + pos.first;
+        ns[c] = __ldg(J + i * pos.stride) + __ldg(J + k * pos.stride);
+      }
+      line_pair_flux<DIM, VF, MEAN_GENERAL>(L, Q, ns, p->inv_gm1, nullptr, f);
+      const double dik = __dmul_rn(scale, p->basis.Dvol[i][k]);
+      const double dki = __dmul_rn(scale, p->basis.Dvol[k][i]);
 #pragma unroll
-        for (int c = 0; c < DIM; ++c)
-          nrm[c] = __ldg(M.tab.fv[dir][c] + (int64_t)E.row[c] * (N - 1) * NF + (m - 1) * NF + line);
-        line_llf<DIM>(L, S, nrm, f);
-        const double wl = alpha * p.basis.inv_w[m - 1], wr = -alpha * p.basis.inv_w[m];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-          acc[m - 1][v] = __fma_rn(wl, f[v], acc[m - 1][v]);
-          acc[m][v] = __fma_rn(wr, f[v], acc[m][v]);
-        }
-        L = S;
+      for (int v = 0; v < NV; ++v) {
+        R[v * PLANE + oi] = __fma_rn(dik, f[v], R[v * PLANE + oi]);
+        R[v * PLANE + ok] = __fma_rn(dki, f[v], R[v * PLANE + ok]);
       }
     }
   }
+}
 
-  // surface fluxes at both ends of the line, lifted into its end nodes
-  // (surface_flux.hpp:45-271, surface_integral.hpp:35-154)
+// Volume term of a line.  Returns 0, or for a line outside the short series'
+// range 1 (long series) or 2 (general means); acc is then zero and the caller
+// adds the term with line_volume_steep after everything else.
+template <int DIM, int N, int VF, bool XL>
+__device__ __forceinline__ int line_volume(const StageArgs<N>& p, const LinePos<DIM, N>& pos,
+                                           const double* P, const double (*ja)[DIM],
+                                           LineNode<DIM>* q, double (*acc)[DIM + 2]) {
+  line_nodes<DIM, N, VF, XL>(P, pos, q);
+  const int range = line_pairs<DIM, N, VF, MEAN_SHORT>(p, q, ja, acc);
+  constexpr int kShortRange = 0x3f1a36e2, kLongRange = 0x3fb00000;  // high words: 1e-4, 1/16
+  if (VF == VF_KENNEDY_GRUBER || range < kShortRange) return 0;
+#pragma unroll
+  for (int m = 0; m < N; ++m)
+#pragma unroll
+    for (int v = 0; v < DIM + 2; ++v) acc[m][v] = 0.0;
+  return range < kLongRange ? 1 : 2;
+}
+
+// Shock-capturing blend of a troubled line (volume_flux.hpp:817-842): (1 -
+// alpha) DG + alpha FV, the FV subcell fluxes (:457-509 in 2D, :521-630 in 3D)
+// once per interface.
+template <int DIM, int N, int VF>
+__device__ __forceinline__ void line_blend(const StageArgs<N>& p, const MeshView& M,
+                                           const LineElement<DIM>& E, int dir, int line,
+                                           const LinePos<DIM, N>& pos, const double* P,
+                                           double alpha, double (*acc)[DIM + 2]) {
+  using G = LineGeo<DIM, N>;
+  using K = LineSlots<DIM, VF>;
+  constexpr int NV = G::NV, NF = G::NF, PLANE = G::PLANE;
+  const double one_m = 1.0 - alpha;
+#pragma unroll
+  for (int m = 0; m < N; ++m)
+#pragma unroll
+    for (int v = 0; v < NV; ++v) acc[m][v] = __dmul_rn(acc[m][v], one_m);
+  auto node = [&](int m) {
+    LineFace<DIM> s;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) s.u[v] = P[v * PLANE + pos.off[m]];
+    const double hinv = P[K::HINV * PLANE + pos.off[m]];
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) s.hv[d] = __dmul_rn(s.u[1 + d], hinv);
+    s.p = P[K::P * PLANE + pos.off[m]];
+    s.qa2 = __dmul_rn(__dmul_rn(0.5 * p.gamma, s.p), hinv);
+    return s;
+  };
+  LineFace<DIM> L = node(0);
+#pragma unroll
+  for (int m = 1; m < N; ++m) {
+    const LineFace<DIM> S = node(m);
+    double nrm[DIM], f[NV];
+#pragma unroll
+    for (int c = 0; c < DIM; ++c)
+      nrm[c] = __ldg(M.tab.fv[dir][c] + (int64_t)E.row[c] * (N - 1) * NF + (m - 1) * NF + line);
+    line_llf<DIM>(L, S, nrm, f);
+    const double wl = alpha * p.basis.inv_w[m - 1], wr = -alpha * p.basis.inv_w[m];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      acc[m - 1][v] = __fma_rn(wl, f[v], acc[m - 1][v]);
+      acc[m][v] = __fma_rn(wr, f[v], acc[m][v]);
+    }
+    L = S;
+  }
+}
+
+// Surface fluxes at both ends of a line (surface_flux.hpp:45-271): `take(s, f)`
+// receives the flux of the low (s = 0) and the high face.  jlo, nh: normals of
+// the low and high face; tr: far states, at boundary faces of 2D meshes
+// replaced by the boundary states.
+template <int DIM, int N, int VF, int SF, class Take>
+__device__ __forceinline__ void line_faces(const StageArgs<N>& p, const MeshView& M,
+                                           const LineElement<DIM>& E, int dir,
+                                           const LinePos<DIM, N>& pos, const double* P,
+                                           const int* nb, double (*tr)[DIM + 2],
+                                           const double* jlo, const double* nh, double t_stage,
+                                           Take&& take) {
+  using K = LineSlots<DIM, VF>;
+  constexpr int NV = DIM + 2, PLANE = LineGeo<DIM, N>::PLANE;
+  const double gamma = p.gamma;
   if constexpr (DIM == 2) {
     if ((nb[0] | nb[1]) < 0) {
 #pragma unroll 1
@@ -642,9 +709,9 @@ __device__ __forceinline__ void line_sweep(const StageArgs<N>& p, const MeshView
         if ((s ? nb[1] : nb[0]) >= 0) continue;
         double ui[NV], ux[NV], nrm[DIM];
 #pragma unroll
-        for (int v = 0; v < NV; ++v) ui[v] = s ? end[1][v] : end[0][v];
+        for (int v = 0; v < NV; ++v) ui[v] = P[v * PLANE + (s ? pos.off[N - 1] : pos.off[0])];
 #pragma unroll
-        for (int c = 0; c < DIM; ++c) nrm[c] = s ? nh[c] : ja[0][c];
+        for (int c = 0; c < DIM; ++c) nrm[c] = s ? nh[c] : jlo[c];
         line_boundary_state<N>(p, M, E, pos, P, 2 * dir + s, t_stage, ui, nrm, ux);
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
@@ -657,111 +724,158 @@ __device__ __forceinline__ void line_sweep(const StageArgs<N>& p, const MeshView
   auto face = [&](int s) {
     LineFace<DIM> own, far;
     double nrm[DIM], f[NV];
+    const int o = s ? pos.off[N - 1] : pos.off[0];
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-      own.u[v] = s ? end[1][v] : end[0][v];
+      own.u[v] = P[v * PLANE + o];
       far.u[v] = s ? tr[1][v] : tr[0][v];
     }
 #pragma unroll
-    for (int c = 0; c < DIM; ++c) nrm[c] = s ? nh[c] : ja[0][c];
+    for (int c = 0; c < DIM; ++c) nrm[c] = s ? nh[c] : jlo[c];
     if constexpr (!(SF == SF_HLLC && DIM == 2)) {
+      const double hinv = P[K::HINV * PLANE + o];
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) own.hv[d] = s ? q[N - 1].hv[d] : q[0].hv[d];
-      own.p = s ? q[N - 1].p : q[0].p;
-      own.qa2 = __dmul_rn(__dmul_rn(0.5 * gamma, own.p), s ? ehinv[1] : ehinv[0]);
+      for (int d = 0; d < DIM; ++d) own.hv[d] = __dmul_rn(own.u[1 + d], hinv);
+      own.p = P[K::P * PLANE + o];
+      own.qa2 = __dmul_rn(__dmul_rn(0.5 * gamma, own.p), hinv);
       line_face_prepare<DIM>(far, gamma);
     }
-    if (s) {
+    // own state left of the face at the high end, right of it at the low end
+    if (s)
       line_surface_flux<DIM, SF>(own, far, nrm, gamma, f);
-#pragma unroll
-      for (int v = 0; v < NV; ++v) acc[N - 1][v] = __fma_rn(f[v], p.basis.lhat_rN, acc[N - 1][v]);
-    } else {
+    else
       line_surface_flux<DIM, SF>(far, own, nrm, gamma, f);
-#pragma unroll
-      for (int v = 0; v < NV; ++v) acc[0][v] = __fma_rn(-f[v], p.basis.lhat_l0, acc[0][v]);
-    }
+    take(s, f);
   };
   if constexpr (SF == SF_HLLC && DIM == 2) {
-    // the longer flux once, for both ends in turn (own state left of the face
-    // at the high end, right of it at the low end)
+    // the longer flux once, for both ends in turn
 #pragma unroll 1
     for (int s = 0; s < 2; ++s) {
       LineFace<DIM> l, r;
       double nrm[DIM], f[NV];
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
-        l.u[v] = s ? end[1][v] : tr[0][v];
-        r.u[v] = s ? tr[1][v] : end[0][v];
+        const double own = P[v * PLANE + (s ? pos.off[N - 1] : pos.off[0])];
+        l.u[v] = s ? own : tr[0][v];
+        r.u[v] = s ? tr[1][v] : own;
       }
 #pragma unroll
-      for (int c = 0; c < DIM; ++c) nrm[c] = s ? nh[c] : ja[0][c];
+      for (int c = 0; c < DIM; ++c) nrm[c] = s ? nh[c] : jlo[c];
       line_surface_flux<DIM, SF>(l, r, nrm, gamma, f);
-#pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        acc[0][v] = __fma_rn(-f[v], s ? 0.0 : p.basis.lhat_l0, acc[0][v]);
-        acc[N - 1][v] = __fma_rn(f[v], s ? p.basis.lhat_rN : 0.0, acc[N - 1][v]);
-      }
+      take(s, f);
     }
   } else {
     face(0);
     face(1);
   }
+}
 
-  if constexpr (NS) {
-    // viscous terms, outside the shock-capturing blend (the reference adds
-    // the parabolic terms separately, structured_solver.hpp:437-480): Dhat
-    // product of the contravariant flux along the line (parabolic_viscous.hpp:
-    // 398-466) and the one-sided interface fluxes of the high-side elements,
-    // the line's own at its low end (br1_kernel.cuh)
-    constexpr int NQ = DIM + 1;
-    const double* V = p.visc + ((int64_t)E.e * DIM + dir) * (NQ * ND) + pos.first;
-    const double* Vn = p.visc + ((int64_t)max(nb[1], 0) * DIM + dir) * (NQ * ND) + pos.first;
-    bool lo = true, hi = true;
-    if (DIM == 2 && (nb[0] | nb[1]) < 0) {
-      // no-slip walls: the inner flux on the momentum rows; slip walls: none
-      lo = nb[0] >= 0 || p.bc.kind[2 * dir] == BC_NS_NOSLIP_ADIABATIC_WALL;
-      hi = nb[1] >= 0 || p.bc.kind[2 * dir + 1] == BC_NS_NOSLIP_ADIABATIC_WALL;
-    }
+// Lifts a face flux into the line's end node (surface_integral.hpp:35-154).
+template <int N, int NV>
+__device__ __forceinline__ void line_lift(const StageArgs<N>& p, int s, const double* f,
+                                          double (*acc)[NV]) {
 #pragma unroll
-    for (int r = 0; r < NQ; ++r) {
-      double w[N];
-      if constexpr (XL) {
-        load_xline<N, true>(V + r * ND, w);
-      } else {
-#pragma unroll
-        for (int m = 0; m < N; ++m) w[m] = __ldg(V + r * ND + m * pos.stride);
-      }
-      double wl = w[0], wh = __ldg(Vn + r * ND);
-      if constexpr (DIM == 2) {
-        wh = nb[1] >= 0 ? wh : w[N - 1];
-        wl = !lo || (nb[0] < 0 && r == DIM) ? 0.0 : wl;
-        wh = !hi || (nb[1] < 0 && r == DIM) ? 0.0 : wh;
-      }
-#pragma unroll
-      for (int m = 0; m < N; ++m)
-#pragma unroll
-        for (int k = 0; k < N; ++k)
-          acc[m][1 + r] = __fma_rn(p.basis.Dhat[m][k], w[k], acc[m][1 + r]);
-      acc[0][1 + r] = __fma_rn(-wl, p.basis.lhat_l0, acc[0][1 + r]);
-      acc[N - 1][1 + r] = __fma_rn(wh, p.basis.lhat_rN, acc[N - 1][1 + r]);
-    }
+  for (int v = 0; v < NV; ++v) {
+    acc[0][v] = s ? acc[0][v] : __fma_rn(-f[v], p.basis.lhat_l0, acc[0][v]);
+    acc[N - 1][v] = s ? __fma_rn(f[v], p.basis.lhat_rN, acc[N - 1][v]) : acc[N - 1][v];
   }
+}
 
-  // add to R
-  const bool read = dir > 0 || (VF != VF_KENNEDY_GRUBER && outside);
+// Viscous terms of a line, outside the shock-capturing blend (the reference
+// adds the parabolic terms separately, structured_solver.hpp:437-480): Dhat
+// product of the contravariant flux along the line (parabolic_viscous.hpp:
+// 398-466) and the one-sided interface fluxes of the high-side elements, the
+// line's own at its low end (br1_kernel.cuh).
+template <int DIM, int N, bool XL>
+__device__ __forceinline__ void line_viscous(const StageArgs<N>& p, const LineElement<DIM>& E,
+                                             int dir, const LinePos<DIM, N>& pos, const int* nb,
+                                             double (*acc)[DIM + 2]) {
+  constexpr int NQ = DIM + 1, ND = LineGeo<DIM, N>::ND;
+  const double* V = p.visc + ((int64_t)E.e * DIM + dir) * (NQ * ND) + pos.first;
+  const double* Vn = p.visc + ((int64_t)max(nb[1], 0) * DIM + dir) * (NQ * ND) + pos.first;
+  bool lo = true, hi = true;
+  if (DIM == 2 && (nb[0] | nb[1]) < 0) {
+    // no-slip walls: the inner flux on the momentum rows; slip walls: none
+    lo = nb[0] >= 0 || p.bc.kind[2 * dir] == BC_NS_NOSLIP_ADIABATIC_WALL;
+    hi = nb[1] >= 0 || p.bc.kind[2 * dir + 1] == BC_NS_NOSLIP_ADIABATIC_WALL;
+  }
+#pragma unroll
+  for (int r = 0; r < NQ; ++r) {
+    double w[N];
+    if constexpr (XL) {
+      load_xline<N, true>(V + r * ND, w);
+    } else {
+#pragma unroll
+      for (int m = 0; m < N; ++m) w[m] = __ldg(V + r * ND + m * pos.stride);
+    }
+    double wl = w[0], wh = __ldg(Vn + r * ND);
+    if constexpr (DIM == 2) {
+      wh = nb[1] >= 0 ? wh : w[N - 1];
+      wl = !lo || (nb[0] < 0 && r == DIM) ? 0.0 : wl;
+      wh = !hi || (nb[1] < 0 && r == DIM) ? 0.0 : wh;
+    }
+#pragma unroll
+    for (int m = 0; m < N; ++m)
+#pragma unroll
+      for (int k = 0; k < N; ++k)
+        acc[m][1 + r] = __fma_rn(p.basis.Dhat[m][k], w[k], acc[m][1 + r]);
+    acc[0][1 + r] = __fma_rn(-wl, p.basis.lhat_l0, acc[0][1 + r]);
+    acc[N - 1][1 + r] = __fma_rn(wh, p.basis.lhat_rN, acc[N - 1][1 + r]);
+  }
+}
+
+// One direction of a lane's line; its contribution is added to R (written by
+// the first direction).
+template <int DIM, int N, int VF, int SF, bool HG, bool NS, bool XL>
+__device__ __forceinline__ void line_sweep(const StageArgs<N>& p, const MeshView& M,
+                                           const LineElement<DIM>& E, int dir, int el, int line,
+                                           const double* P, double* R, double alpha,
+                                           double t_stage) {
+  constexpr int NV = DIM + 2, PLANE = LineGeo<DIM, N>::PLANE;
+  LinePos<DIM, N> pos;
+  pos.set(dir, el, line);
+  // the direction's global loads, requested together before the volume term
+  int nb[2];
+  double ja[N][DIM], nh[DIM], tr[2][NV], acc[N][NV];
+  line_metrics<DIM, N, XL>(M, E, dir, pos, ja);
+  line_ends<DIM, N>(M, E, dir, pos, nb, nh);
+  line_traces<DIM, N>(M, pos, nb, tr);
+  LineNode<DIM> q[N];
+  const int steep = line_volume<DIM, N, VF, XL>(p, pos, P, ja, q, acc);
+  const bool troubled = HG && fabs(alpha - 0.0) > p.atol;
+  if constexpr (HG) {
+    if (troubled)
+      line_blend<DIM, N, VF>(p, M, E, dir, line, pos, P, alpha, acc);
+  }
+  line_faces<DIM, N, VF, SF>(p, M, E, dir, pos, P, nb, tr, ja[0], nh, t_stage,
+                             [&](int s, const double* f) { line_lift<N, NV>(p, s, f, acc); });
+  if constexpr (NS) line_viscous<DIM, N, XL>(p, E, dir, pos, nb, acc);
+  if (steep) {
+    // the direction's terms in R, R's former line in acc
+#pragma unroll
+    for (int v = 0; v < NV; ++v)
+#pragma unroll
+      for (int m = 0; m < N; ++m) {
+        double* r = R + v * PLANE + pos.off[m];
+        const double t = *r;
+        *r = acc[m][v];
+        acc[m][v] = t;
+      }
+    line_volume_steep<DIM, N, VF>(&p, &M, E, dir, el, line, P, R, steep == 1,
+                                  troubled ? 1.0 - alpha : 1.0);
+  }
+  if (steep && dir == 0) return;
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
     double r[N];
-    if (read) {
+    if (dir > 0) {
       load_line<XL, N>(R + v * PLANE, pos.off, r);
 #pragma unroll
       for (int m = 0; m < N; ++m) acc[m][v] += r[m];
     }
-    if (N % 2 == 0 || dir < DIM - 1) {
 #pragma unroll
-      for (int m = 0; m < N; ++m) r[m] = acc[m][v];
-      store_line<XL, N>(R + v * PLANE, pos.off, r);
-    }
+    for (int m = 0; m < N; ++m) r[m] = acc[m][v];
+    store_line<XL, N>(R + v * PLANE, pos.off, r);
   }
 }
 
@@ -771,6 +885,33 @@ __device__ __forceinline__ void line_sweep(const StageArgs<N>& p, const MeshView
 __device__ __forceinline__ double markstein_div(double a, double b, double y) {
   const double q = __dmul_rn(a, y);
   return __fma_rn(__fma_rn(-q, b, a), y, q);
+}
+
+// Node data published per node: 1 / (2 rho), p, Chandrashekar rho / p, and
+// with shock capturing the indicator variable rho p (hg_node_value[_3d],
+// indicator.hpp:148-161, :187-210, gamma = 1.4, every operation rounded as
+// written there; it needs the correctly rounded reciprocal, see markstein_div).
+template <int DIM, int VF, bool HG>
+__device__ __forceinline__ void line_prepare_node(const double* u, double gamma, double& hinv,
+                                                  double& pr, double& b, double& ind) {
+  const double inv = HG ? 1.0 / u[0] : recip(u[0]);
+  hinv = 0.5 * inv;
+  double hv[DIM];
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) hv[d] = __dmul_rn(u[1 + d], hinv);
+  pr = __dmul_rn(gamma - 1.0, u[DIM + 1] - line_dot<DIM>(u + 1, hv));
+  if constexpr (VF == VF_CHANDRASHEKAR) b = quotient(u[0], pr);
+  if constexpr (HG) {
+    double vv = 0.0;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      const double vd = markstein_div(u[1 + d], u[0], inv);
+      const double v2 = __dmul_rn(vd, vd);
+      vv = d == 0 ? v2 : __dadd_rn(vv, v2);
+    }
+    ind = __dmul_rn(
+        __dmul_rn(1.4 - 1.0, __dsub_rn(u[DIM + 1], __dmul_rn(__dmul_rn(0.5, u[0]), vv))), u[0]);
+  }
 }
 
 // Squared modes of one element in node order, read through a plane.
@@ -853,7 +994,7 @@ __device__ __forceinline__ void stage_line_body(const StageArgs<N>& p) {
   constexpr int EPB = EPW * WPB;
   // Directions share one copy of the code where a copy each would not stay in
   // the instruction cache.
-  constexpr bool ROLL = N > 4 || HG || SF == SF_HLLC;
+  constexpr bool ROLL = N > 4;
   constexpr bool XSTORE = N % 2 == 0;  // store by x lines
   extern __shared__ __align__(128) double smem_line[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -911,31 +1052,10 @@ __device__ __forceinline__ void stage_line_body(const StageArgs<N>& p) {
     double hinv[N], pr[N], b[N];
 #pragma unroll
     for (int m = 0; m < N; ++m) {
-      // shock capturing needs the correctly rounded reciprocal (markstein_div)
-      const double inv = HG ? 1.0 / u[0][m] : recip(u[0][m]);
-      hinv[m] = 0.5 * inv;
-      double ke = 0.0;
+      double un[NV];
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) {
-        const double hv = __dmul_rn(u[1 + d][m], hinv[m]);
-        ke = d == 0 ? __dmul_rn(u[1 + d][m], hv) : __fma_rn(u[1 + d][m], hv, ke);
-      }
-      pr[m] = __dmul_rn(gamma - 1.0, u[NV - 1][m] - ke);
-      if constexpr (VF == VF_CHANDRASHEKAR) b[m] = quotient(u[0][m], pr[m]);
-      if constexpr (HG) {
-        // hg_node_value[_3d] (indicator.hpp:148-161, :187-210), gamma = 1.4
-        double vv = 0.0;
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) {
-          const double vd = markstein_div(u[1 + d][m], u[0][m], inv);
-          const double v2 = __dmul_rn(vd, vd);
-          vv = d == 0 ? v2 : __dadd_rn(vv, v2);
-        }
-        ind[m] = __dmul_rn(
-            __dmul_rn(1.4 - 1.0,
-                      __dsub_rn(u[NV - 1][m], __dmul_rn(__dmul_rn(0.5, u[0][m]), vv))),
-            u[0][m]);
-      }
+      for (int v = 0; v < NV; ++v) un[v] = u[v][m];
+      line_prepare_node<DIM, VF, HG>(un, gamma, hinv[m], pr[m], b[m], ind[m]);
     }
 #pragma unroll
     for (int v = 0; v < NV; ++v) store_line<true, N>(P + v * PLANE, pos.off, u[v]);
@@ -947,26 +1067,22 @@ __device__ __forceinline__ void stage_line_body(const StageArgs<N>& p) {
   if constexpr (HG) alpha = line_alpha<DIM, N>(p, R, el, line, act, E.e, ind);
 
   // ---- directions ------------------------------------------------------------
-  double acc[N][NV];
-  LinePos<DIM, N> pos;
   if constexpr (ROLL) {
 #pragma unroll 1
     for (int dir = 0; dir < DIM; ++dir) {
       __syncwarp();
       if (act)
-        line_sweep<DIM, N, VF, SF, HG, NS, false>(p, M, E, dir, el, line, P, R, alpha, t_stage, acc,
-                                              pos);
+        line_sweep<DIM, N, VF, SF, HG, NS, false>(p, M, E, dir, el, line, P, R, alpha, t_stage);
     }
   } else {
     __syncwarp();
     if (act)
-      line_sweep<DIM, N, VF, SF, HG, NS, true>(p, M, E, 0, el, line, P, R, alpha, t_stage, acc, pos);
+      line_sweep<DIM, N, VF, SF, HG, NS, true>(p, M, E, 0, el, line, P, R, alpha, t_stage);
 #pragma unroll
     for (int dir = 1; dir < DIM; ++dir) {
       __syncwarp();
       if (act)
-        line_sweep<DIM, N, VF, SF, HG, NS, false>(p, M, E, dir, el, line, P, R, alpha, t_stage, acc,
-                                              pos);
+        line_sweep<DIM, N, VF, SF, HG, NS, false>(p, M, E, dir, el, line, P, R, alpha, t_stage);
     }
   }
   __syncwarp();
@@ -977,7 +1093,8 @@ __device__ __forceinline__ void stage_line_body(const StageArgs<N>& p) {
     bool bad = false;
     double mij[N], un[NV][N], vals[N][NV];
     const double* mij_e = M.mij + (int64_t)E.e * ND;
-    if constexpr (XSTORE) pos.set(0, el, line);
+    LinePos<DIM, N> pos;
+    pos.set(XSTORE ? 0 : DIM - 1, el, line);
     if constexpr (XSTORE) {
       load_xline<N, true>(mij_e + pos.first, mij);
       if (p.a != 0.0) {
@@ -1001,19 +1118,17 @@ __device__ __forceinline__ void stage_line_body(const StageArgs<N>& p) {
             un[v][m] = M.u_n[ebase + v * ND + pos.first + m * pos.stride];
       }
     }
+    double cm[N];
+#pragma unroll
+    for (int m = 0; m < N; ++m) cm[m] = __dmul_rn(M.c, mij[m]);
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
       double r[N], ui[N];
-      if constexpr (XSTORE) {
-        load_line<true, N>(R + v * PLANE, pos.off, r);
-      } else {
-#pragma unroll
-        for (int m = 0; m < N; ++m) r[m] = acc[m][v];
-      }
+      load_line<XSTORE, N>(R + v * PLANE, pos.off, r);
       if (p.b != 0.0) load_line<XSTORE, N>(P + v * PLANE, pos.off, ui);
 #pragma unroll
       for (int m = 0; m < N; ++m) {
-        double val = __dmul_rn(M.c, __dmul_rn(r[m], mij[m]));
+        double val = __dmul_rn(r[m], cm[m]);
         if (p.b != 0.0) val = __fma_rn(p.b, ui[m], val);
         if (p.a != 0.0) val = __fma_rn(p.a, un[v][m], val);
         bad |= !isfinite(val);
@@ -1056,8 +1171,253 @@ __device__ __forceinline__ void stage_line_body(const StageArgs<N>& p) {
 
 // MINB resident blocks per SM are requested from the register allocator.
 template <int DIM, int N, int VF, int SF, bool HG, bool NS, bool BATCH, int WPB, int MINB>
-__global__ void __launch_bounds__(32 * WPB, MINB) stage_line_kernel(const StageArgs<N> p) {
+__global__ void __launch_bounds__(32 * WPB, MINB) stage_line_kernel(const __grid_constant__ StageArgs<N> p) {
   stage_line_body<DIM, N, VF, SF, HG, NS, BATCH, WPB>(p);
+}
+
+// ---------------------------------------------------------------------------
+// The same arithmetic with a block per group of EPW elements, for meshes that
+// do not fill the GPU with one warp per group: the warps of the block take
+//   load   the group's nodes, one per thread;
+//   sweep  warp d < DIM: volume term of direction d; warp DIM + d: the face
+//          fluxes of direction d (into F); with shock capturing one more warp:
+//          alpha; then warp d: blend, lifting, viscous terms -> its planes R_d;
+//   store  the group's nodes, one per thread: R_0 + R_1 [+ R_2], -1/J, SSPRK3
+//          combination.
+// The chain of dependent instructions of a lane is a third of the line
+// sweep's; every sum is formed in the same order, so the results are the line
+// sweep's bit for bit.
+// ---------------------------------------------------------------------------
+template <int DIM, int N, int VF, bool HG>
+struct SplitShape {
+  using G = LineGeo<DIM, N>;
+  static constexpr int WARPS = 2 * DIM + (HG ? 1 : 0);
+  static constexpr int NT = 32 * WARPS;
+  static constexpr int NS = LineSlots<DIM, VF>::NS;
+  static constexpr int FACE = 32 * G::NV;  // one (direction, side): [var][lane]
+  static constexpr int DOUBLES = (NS + DIM * G::NV + (HG ? 1 : 0)) * G::PLANE + DIM * 2 * FACE;
+  static constexpr size_t smem_bytes = sizeof(double) * (size_t)DOUBLES;
+  static_assert(!HG || G::EPW <= 16, "alpha per element");
+};
+
+template <int DIM, int N, int VF, int SF, bool HG, bool NS, bool BATCH>
+__device__ __forceinline__ void stage_split_body(const StageArgs<N>& p) {
+  using G = LineGeo<DIM, N>;
+  using K = LineSlots<DIM, VF>;
+  using S = SplitShape<DIM, N, VF, HG>;
+  constexpr int NV = G::NV, ND = G::ND, NF = G::NF, EPW = G::EPW, PLANE = G::PLANE, NT = S::NT;
+  constexpr int PASSES = (EPW * ND + NT - 1) / NT;
+  extern __shared__ __align__(128) double smem_split[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double* P = smem_split;
+  double* R = P + K::NS * PLANE;                  // [dir][var]
+  double* F = R + DIM * NV * PLANE;               // [dir][side][var][lane]
+  double* I = F + DIM * 2 * S::FACE;              // indicator plane (HG)
+  __shared__ double alpha_s[HG ? EPW : 1];
+
+  __shared__ MeshView mesh_s;
+  int e0;
+  // tables are read before the wait (see stage_line_body)
+  if constexpr (BATCH) {
+    static_assert(NT >= int(sizeof(MeshView) / 8), "block narrower than the mesh view");
+    e0 = p.tile_e0[blockIdx.x];
+    copy_mesh_view(&mesh_s, p.meshes, p.tile_mesh[blockIdx.x], tid);
+    __syncthreads();
+  } else {
+    e0 = (int)blockIdx.x * EPW;
+  }
+  const MeshView& M = BATCH ? mesh_s : p.mesh;
+  const int ne = min(EPW, M.nelem - e0);
+  const int el = lane / NF, line = lane - el * NF;
+  const bool act = el < ne;
+  const int dir = warp % DIM;
+  const bool volume = warp < DIM, faces = !volume && warp < 2 * DIM;
+  LineElement<DIM> E;
+  E.e = act ? e0 + el : e0;
+  E.info = M.info + (int64_t)E.e * 12;
+#pragma unroll
+  for (int c = 0; c < DIM; ++c) E.row[c] = __ldg(E.info + 3 + c);
+  LinePos<DIM, N> pos;
+  pos.set(dir, el, line);
+  int nb[2];
+  double ja[N][DIM], nh[DIM], tr[2][NV];
+  if (volume) {
+    line_metrics<DIM, N, false>(M, E, dir, pos, ja);
+    nb[0] = __ldg(E.info + 6 + 2 * dir);
+    nb[1] = __ldg(E.info + 7 + 2 * dir);
+  } else if (faces) {
+    line_ends<DIM, N>(M, E, dir, pos, nb, nh);
+#pragma unroll
+    for (int c = 0; c < DIM; ++c)
+      ja[0][c] = __ldg(M.tab.ja[dir][c] + (int64_t)E.row[c] * ND + pos.first);
+  }
+  stage_dependency_sync();
+  const double gamma = p.gamma;
+  const double t_stage = p.t_dev ? (*p.t_dev + p.t) : p.t;
+  const int64_t gbase = (int64_t)e0 * (NV * ND);
+  const bool with_n = p.a != 0.0;
+
+  // ---- load, node data, publish --------------------------------------------
+  int opos[PASSES];
+#pragma unroll
+  for (int k = 0; k < PASSES; ++k) {
+    const int t = tid + k * NT, te = t / ND, node = t - te * ND;
+    opos[k] = te < ne ? LinePos<DIM, N>::slot(0, te, node / N, node % N) : -1;
+    if (opos[k] < 0) continue;
+    const int o = opos[k];
+    double u[NV], hinv, pr, b = 0.0, ind = 0.0;
+    const double* src = M.u_in + gbase + (int64_t)te * (NV * ND) + node;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) u[v] = __ldg(src + v * ND);
+    line_prepare_node<DIM, VF, HG>(u, gamma, hinv, pr, b, ind);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) P[v * PLANE + o] = u[v];
+    P[K::HINV * PLANE + o] = hinv;
+    P[K::P * PLANE + o] = pr;
+    if constexpr (VF == VF_CHANDRASHEKAR) P[K::B * PLANE + o] = b;
+    if constexpr (HG) I[o] = ind;
+  }
+  if (faces) line_traces<DIM, N>(M, pos, nb, tr);
+  __syncthreads();
+
+  // ---- volume terms, face fluxes, alpha --------------------------------------
+  double acc[N][NV];
+  int steep = 0;
+  double* Rd = R + dir * (NV * PLANE);
+  if (volume) {
+    if (act) {
+      LineNode<DIM> q[N];
+      steep = line_volume<DIM, N, VF, false>(p, pos, P, ja, q, acc);
+      // A steep line's term in straight code right here (this kernel's chain is
+      // short: the call of line_volume_steep cost KH 64^2 1.0 of 5.8 us), kept
+      // in R_d until the other terms are there: the same sum in the same order.
+      // Long lines take the call at the end like the line sweep.
+      if ((steep == 1 && N <= (DIM == 2 ? 6 : 4)) || (steep == 2 && N <= 4)) {
+        // copies the compiler cannot relate to the first pass, or it would
+        // keep that pass's intermediate values in registers
+#pragma unroll
+        for (int m = 0; m < N; ++m) {
+          asm volatile("" : "+d"(q[m].rho), "+d"(q[m].p), "+d"(q[m].x), "+d"(q[m].y));
+#pragma unroll
+          for (int d = 0; d < DIM; ++d) asm volatile("" : "+d"(q[m].hv[d]), "+d"(ja[m][d]));
+        }
+        if constexpr (N <= (DIM == 2 ? 6 : 4)) {
+          if (steep == 1)
+            line_pairs<DIM, N, VF, MEAN_LONG>(p, q, ja, acc);
+          else if constexpr (N <= 4)
+            line_pairs<DIM, N, VF, MEAN_GENERAL>(p, q, ja, acc);
+        }
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+#pragma unroll
+          for (int m = 0; m < N; ++m) {
+            Rd[v * PLANE + pos.off[m]] = acc[m][v];
+            acc[m][v] = 0.0;
+          }
+        steep = 4;
+      }
+    }
+  } else if (faces) {
+    if (act)
+      line_faces<DIM, N, VF, SF>(p, M, E, dir, pos, P, nb, tr, ja[0], nh, t_stage,
+                                 [&](int s, const double* f) {
+#pragma unroll
+                                   for (int v = 0; v < NV; ++v)
+                                     F[(dir * 2 + s) * S::FACE + v * 32 + lane] = f[v];
+                                 });
+  } else if constexpr (HG) {
+    double ind[N];
+    LinePos<DIM, N> px;
+    px.set(0, el, line);
+    if (act) load_line<true, N>(I, px.off, ind);
+    const double a = line_alpha<DIM, N>(p, I, el, line, act, E.e, ind);
+    if (act && line == 0) alpha_s[el] = a;
+  }
+  // u_n and -1/J of the thread's nodes, on their way during the barrier
+  double un[PASSES][NV], mij[PASSES];
+#pragma unroll
+  for (int k = 0; k < PASSES; ++k) {
+    if (opos[k] < 0) continue;
+    const int t = tid + k * NT, te = t / ND, node = t - te * ND;
+    mij[k] = __ldg(M.mij + (int64_t)e0 * ND + t);
+    if (with_n) {
+#pragma unroll
+      for (int v = 0; v < NV; ++v)
+        un[k][v] = M.u_n[gbase + (int64_t)te * (NV * ND) + v * ND + node];
+    }
+  }
+  __syncthreads();
+  if (volume && act) {
+    const double alpha = HG ? alpha_s[el] : 0.0;
+    const bool troubled = HG && fabs(alpha - 0.0) > p.atol;
+    if constexpr (HG) {
+      if (troubled)
+        line_blend<DIM, N, VF>(p, M, E, dir, line, pos, P, alpha, acc);
+    }
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      double f[NV];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) f[v] = F[(dir * 2 + s) * S::FACE + v * 32 + lane];
+      line_lift<N, NV>(p, s, f, acc);
+    }
+    if constexpr (NS) line_viscous<DIM, N, false>(p, E, dir, pos, nb, acc);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      double r[N];
+#pragma unroll
+      for (int m = 0; m < N; ++m)
+        r[m] = steep == 4
+                   ? __fma_rn(troubled ? 1.0 - alpha : 1.0, Rd[v * PLANE + pos.off[m]], acc[m][v])
+                   : acc[m][v];
+      store_line<false, N>(Rd + v * PLANE, pos.off, r);
+    }
+    if (steep == 1 || steep == 2)
+      line_volume_steep<DIM, N, VF>(&p, &M, E, dir, el, line, P, Rd, steep == 1,
+                                    troubled ? 1.0 - alpha : 1.0);
+  }
+  __syncthreads();
+
+  // ---- -1/J, SSPRK3 combination, store -----------------------------------------
+  double dacc[3] = {0.0, 0.0, 0.0};
+  bool bad = false;
+#pragma unroll
+  for (int k = 0; k < PASSES; ++k) {
+    const int o = opos[k];
+    if (o < 0) continue;
+    const int t = tid + k * NT, te = t / ND, node = t - te * ND;
+    const double cm = __dmul_rn(M.c, mij[k]);
+    double vals[NV];
+    double* dst = M.out + gbase + (int64_t)te * (NV * ND) + node;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      double r = R[v * PLANE + o];
+#pragma unroll
+      for (int d = 1; d < DIM; ++d) r = R[(d * NV + v) * PLANE + o] + r;
+      double val = __dmul_rn(r, cm);
+      if (p.b != 0.0) val = __fma_rn(p.b, P[v * PLANE + o], val);
+      if (with_n) val = __fma_rn(p.a, un[k][v], val);
+      bad |= !isfinite(val);
+      dst[v * ND] = val;
+      vals[v] = val;
+    }
+    if constexpr (!BATCH) {
+      if (p.diag) diag_add_node<DIM, N>(vals, p.basis, node, -mij[k], gamma, p.inv_gm1, dacc);
+    }
+  }
+  if (bad) atomicOr(p.nonfinite, 1u);
+  if constexpr (!BATCH) {
+    if (p.diag) {
+      __shared__ double red[3 * S::WARPS];
+      diag_block_store<NT>(dacc, red, p.diag + 3 * (int64_t)blockIdx.x);
+    }
+  }
+}
+
+template <int DIM, int N, int VF, int SF, bool HG, bool NS, bool BATCH, int MINB>
+__global__ void __launch_bounds__(SplitShape<DIM, N, VF, HG>::NT, MINB)
+    stage_split_kernel(const __grid_constant__ StageArgs<N> p) {
+  stage_split_body<DIM, N, VF, SF, HG, NS, BATCH>(p);
 }
 
 }  // namespace dgsem

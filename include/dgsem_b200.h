@@ -296,7 +296,8 @@ dgsem_status dgsem_check_finite(dgsem_ctx* ctx);
 
 /* Launch-shape autotuner (no reference counterpart; the reference has one
  * fixed Kokkos launch shape).  The fused stage kernel has up to 7 launch
- * shapes: 0-2 line sweeps (warps per block, register cap), 3-4
+ * shapes: 0-2 line shapes (0 = split over a block or one warp per group of
+ * elements, by the mesh's size; 1 = split; 2 = one warp, other register cap), 3-4
  * node-parallel with and without a register cap, 5 persistent node-parallel
  * streaming element tiles through shared memory with bulk copies (no shock
  * capturing or viscous terms; 2D or even n in 3D), 6 node-parallel with two

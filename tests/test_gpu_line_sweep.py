@@ -1,4 +1,4 @@
-"""The line sweeps (launch shapes 0-2) where they can go wrong: meshes whose
+"""The line shapes (0-2: sweep and split form) where they can go wrong: meshes whose
 rows straddle warps and blocks, a single element across (its own neighbour),
 partly filled warps at every degree, steep nodal jumps (the general path of
 the volume term next to lines that stay on the series), and states that are
