@@ -37,9 +37,9 @@ struct NodeState {
 // Newton-Schulz step); a/b from a (1/b) with one residual correction; sqrt by
 // one Goldschmidt step and a residual correction.  Against the correctly
 // rounded results over 1.5e8 random arguments: the reciprocal is one unit in
-// the last place off in 3e-4 of the cases, quotient and root never
-// Arguments must be normal with normal reciprocals: zero,
-// infinite and subnormal ones give a NaN, except that root is 0 below 1e-290.
+// the last place off in 3e-4 of the cases, quotient and root never.  Arguments
+// must be normal with normal reciprocals: zero, infinite and subnormal ones
+// give a NaN, except that root is 0 below 1e-290.
 // The compiler's division and sqrt carry a branch for those arguments, which
 // ends a scheduling block at every use (node kernels 3-11 % faster without it:
 // DMR stage 23.0 -> 20.6 us, TGV 32^3 Chandrashekar 196 -> 181 us).
