@@ -31,35 +31,45 @@ struct NodeState {
   double inv_rho;
 };
 
-// Branch-free reciprocal, quotient and square root of normal numbers from the
+// Branch-free reciprocals, quotient and square root of normal numbers from the
 // hardware's approximations (rcp.approx.ftz.f64, rsqrt.approx.ftz.f64, about
-// 20 bits): 1/a = r (1 + e + e^2 + O(e^3)) with e = 1 - a r (third-order
-// Newton-Schulz step); a/b from a (1/b) with one residual correction; sqrt by
-// one Goldschmidt step and a residual correction.  Against the correctly
-// rounded results over 1.5e8 random arguments: the reciprocal is one unit in
-// the last place off in 3e-4 of the cases, quotient and root never.  Arguments
-// must be normal with normal reciprocals: zero, infinite and subnormal ones
-// give a NaN, except that root is 0 below 1e-290.
+// 20 bits):
+//   recip_ulp  r (1 + e + e^2) with e = 1 - a r (third-order Newton-Schulz step):
+//              the rounded reciprocal or, in 3e-4 of the cases, its neighbour
+//   recip      r1 + r1 (1 - a r1) with r1 = recip_ulp(a): the rounded reciprocal
+//              (P. Markstein, IBM J. Res. Dev. 34, 1990: every a whose
+//              significand is not all ones)
+//   quotient   q = a (1/b), then q + (a - q b) (1/b) (the same paper)
+//   root       one Goldschmidt step, then g + h (x - g^2)
+// tests/test_gpu_scalar_math.py compares them with the rounded results over
+// random significands and exponents.  Arguments must be normal with normal
+// reciprocals: zero, infinite and subnormal ones give a NaN, except that root
+// is 0 below 1e-290.  So a state with a zero or infinite density (or pressure,
+// where the flux divides by it) gives non-finite values, as with the division.
 // The compiler's division and sqrt carry a branch for those arguments, which
 // ends a scheduling block at every use (node kernels 3-11 % faster without it:
-// DMR stage 23.0 -> 20.6 us, TGV 32^3 Chandrashekar 196 -> 181 us).
-__device__ __forceinline__ double recip(double a) {
+// DMR stage 23.0 -> 20.6 us, TGV 32^3 Chandrashekar 196 -> 181 us; recip's last
+// step, without which it is recip_ulp, costs 0.5-1 % of that).
+__device__ __forceinline__ double recip_ulp(double a) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(a));
   const double e = __fma_rn(-a, r, 1.0);
   return __fma_rn(r, __fma_rn(e, e, e), r);
 }
 
-// One Newton step: relative error about 1e-12.
-__device__ __forceinline__ double recip_approx(double a) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(a));
-  return __fma_rn(r, __fma_rn(-a, r, 1.0), r);
+__device__ __forceinline__ double recip(double a) {
+  const double r1 = recip_ulp(a);
+  return __fma_rn(__fma_rn(-a, r1, 1.0), r1, r1);
+}
+
+// a / b from the rounded reciprocal r = 1 / b.
+__device__ __forceinline__ double quotient_r(double a, double b, double r) {
+  const double q = __dmul_rn(a, r);
+  return __fma_rn(__fma_rn(-q, b, a), r, q);
 }
 
 __device__ __forceinline__ double quotient(double a, double b) {
-  const double r = recip(b), q = __dmul_rn(a, r);
-  return __fma_rn(__fma_rn(-q, b, a), r, q);
+  return quotient_r(a, b, recip(b));
 }
 
 __device__ __forceinline__ double root(double x) {

@@ -230,9 +230,7 @@ struct LineScale {
 
 // How a line evaluates the logarithmic means of its pairs, from f^2 =
 // ((a - b) / (a + b))^2 of both means:
-//   MEAN_SHORT    f^2 < 1e-4: the reference's series (4 terms); the series of
-//                 the mean multiplies f^2 by coefficients of order one, so the
-//                 reciprocal of a + b in f needs 12 digits only
+//   MEAN_SHORT    f^2 < 1e-4: the reference's series (4 terms)
 //   MEAN_LONG     f^2 < 1/16 (a ratio of up to 5/3 between two nodes): the
 //                 same series atanh(f) / f = sum f^2k / (2k + 1) to 13 terms
 //                 (remainder below 1e-17).  The reference takes the logarithm
@@ -240,7 +238,10 @@ struct LineScale {
 //                 the last place; the two agree to that
 //   MEAN_GENERAL  any pair: the reference's rule with the logarithm
 // A line takes the same form for all of its pairs, so each form is one block
-// of straight code.
+// of straight code.  The sums' reciprocals are recip_ulp's (at most 0.501 units
+// in the last place; the node kernels' shared ones, two_reciprocals, 1.5): with
+// rounded ones KH 1024^2 took 503 us per stage instead of 494, a stage of 64
+// batched meshes 694 instead of 674.
 enum LineMean : int { MEAN_SHORT, MEAN_LONG, MEAN_GENERAL };
 
 __device__ __forceinline__ double line_atanh_series(double t) {
@@ -282,18 +283,18 @@ __device__ __forceinline__ void line_pair_flux(const LineNode<DIM>& L, const Lin
     b = __dmul_rn(R.rho, L.p);
   }
   const double s = a + b;
-  const double is = recip(s);
+  const double is = recip_ulp(s);
   double rho_mean, im;
   if constexpr (MEAN == MEAN_GENERAL) {
-    rho_mean = ln_mean_rs(L.rho, R.rho, rs, recip(rs));
+    rho_mean = ln_mean_rs(L.rho, R.rho, rs, recip_ulp(rs));
     im = inv_ln_mean_rs(a, b, is);
   } else if constexpr (MEAN == MEAN_LONG) {
-    const double t = (L.rho - R.rho) * recip(rs), g2 = __dmul_rn(t, t);
+    const double t = (L.rho - R.rho) * recip_ulp(rs), g2 = __dmul_rn(t, t);
     const double w = (a - b) * is, f2 = __dmul_rn(w, w);
-    rho_mean = __dmul_rn(0.5 * rs, recip(line_atanh_series(g2)));
+    rho_mean = __dmul_rn(0.5 * rs, recip_ulp(line_atanh_series(g2)));
     im = __dmul_rn(2.0 * is, line_atanh_series(f2));
   } else {
-    const double t = (L.rho - R.rho) * recip_approx(rs), g2 = __dmul_rn(t, t);
+    const double t = (L.rho - R.rho) * recip_ulp(rs), g2 = __dmul_rn(t, t);
     const double w = (a - b) * is, f2 = __dmul_rn(w, w);
     // both are >= 0 or NaN: compared on the high words, no FP64 compare
     *range = max(*range, max(__double2hiint(g2), __double2hiint(f2)));
@@ -879,18 +880,10 @@ __device__ __forceinline__ void line_sweep(const StageArgs<N>& p, const MeshView
   }
 }
 
-// Correctly rounded a / b from q = a y with the correctly rounded reciprocal
-// y = 1 / b: q + (a - q b) y (Markstein's theorem, IBM J. Res. Dev. 34, 1990;
-// no under- or overflow at the magnitudes of a flow state).
-__device__ __forceinline__ double markstein_div(double a, double b, double y) {
-  const double q = __dmul_rn(a, y);
-  return __fma_rn(__fma_rn(-q, b, a), y, q);
-}
-
 // Node data published per node: 1 / (2 rho), p, Chandrashekar rho / p, and
 // with shock capturing the indicator variable rho p (hg_node_value[_3d],
 // indicator.hpp:148-161, :187-210, gamma = 1.4, every operation rounded as
-// written there; it needs the correctly rounded reciprocal, see markstein_div).
+// written there; quotient_r needs the rounded reciprocal).
 template <int DIM, int VF, bool HG>
 __device__ __forceinline__ void line_prepare_node(const double* u, double gamma, double& hinv,
                                                   double& pr, double& b, double& ind) {
@@ -905,7 +898,7 @@ __device__ __forceinline__ void line_prepare_node(const double* u, double gamma,
     double vv = 0.0;
 #pragma unroll
     for (int d = 0; d < DIM; ++d) {
-      const double vd = markstein_div(u[1 + d], u[0], inv);
+      const double vd = quotient_r(u[1 + d], u[0], inv);
       const double v2 = __dmul_rn(vd, vd);
       vv = d == 0 ? v2 : __dadd_rn(vv, v2);
     }
