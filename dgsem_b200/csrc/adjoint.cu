@@ -47,6 +47,13 @@ class AdjointEngine final : public AdjointEngineBase {
  public:
   static constexpr int EPB = (128 / (N * N)) > 0 ? (128 / (N * N)) : 1;
 
+  // This unit launches viscous_flux_kernel itself, with more than 48 KB of
+  // shared memory from n = 6 on: it does not rely on the forward engine's unit
+  // having configured the same kernel.
+  AdjointEngine() {
+    if constexpr (NS) set_viscous_flux_attributes<2, N>();
+  }
+
   cudaError_t vjp(const EngineConfig& cfg, const double* u, double* grad_u, bool fresh,
                   const double* w, double* out, const double* X, double x0, const double* Y,
                   double x1, double b, double c, double* xy, double* qdir,

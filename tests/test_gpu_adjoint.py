@@ -99,6 +99,31 @@ def test_rhs_vjp_adjoint_identity_adjoint_mesh(cuda):
         assert abs(lhs - rhs) <= 1e-10 * mag, (k, lhs, rhs, mag)
 
 
+@pytest.mark.parametrize("viscous", [True, False])
+@pytest.mark.parametrize("polydeg", range(1, 8))
+def test_rhs_vjp_every_degree_vs_autograd(polydeg, viscous, cuda):
+    """A standalone VJP (the gradient kernel included, whose shared memory grows
+    with the degree) against torch's reverse mode of the 64-bit form of the
+    method in perf/cases.py.  The bar is four times the largest distance seen
+    (8.7e-15 at n = 8; that form takes ideal metrics, the library the reference's
+    rounded ones)."""
+    import torch
+
+    import dgsem_b200 as D
+    from perf import cases as P
+    case = P._case(None, "rhs", "tgv2d", polydeg, 5, 4, 0, "chandrashekar", viscous=viscous)
+    _, _, _, solver = P._solver(case)
+    u = P._state(case, 3, cuda)
+    w = torch.randn(u.shape, generator=torch.Generator().manual_seed(polydeg),
+                    dtype=torch.float64).to(cuda)
+    got = D.Adjoint(solver, 1, 1).rhs_vjp(u, w)
+    leaf = u.clone().requires_grad_(True)
+    (want,) = torch.autograd.grad(P._Method(case, cuda).rhs(leaf, 0.0), leaf, w)
+    err = float((got - want).norm() / want.norm())
+    print(f"\n  n={polydeg + 1} viscous={viscous}: {err:.2e}")
+    assert err <= 4e-14
+
+
 def test_kinetic_energy_matches_oracle(cuda):
     import torch
     s = make_oracle(NS_RECT)
