@@ -6,7 +6,7 @@
 // for each segment, last to first, the segment's steps are recomputed from
 // its checkpoint while their stage states (u^n, u^(1), u^(2)) are kept in
 // HBM (the last segment is recorded during the forward pass and not
-// recomputed), with Navier-Stokes also the BR1 gradient of each of those
+// recomputed), with Navier-Stokes also the velocity gradient of each of those
 // states as the forward stage computed it (so the reverse VJPs do not
 // recompute it), then the adjoint SSPRK3 steps run backwards:
 //   lam2 = 2/3 lam + 2/3 dt VJP(u^(2); lam)
@@ -233,7 +233,7 @@ struct dgsem_adjoint {
   std::vector<void*> allocations;
   double* snaps = nullptr;  // [nsnap][len]
   double* seg = nullptr;    // [every][3][len]: u^n, u^(1), u^(2) of each step
-  // Navier-Stokes: [every][3][glen] forward BR1 gradients of those states,
+  // Navier-Stokes: [every][3][glen] velocity gradients of those states,
   // written by the forward stages that consume them (nullptr: Euler)
   double* gseg = nullptr;
   int64_t glen = 0;
@@ -333,8 +333,8 @@ cudaError_t launch_vjp(dgsem_adjoint* a, const double* u, double* grad_u, const 
   // without a kept gradient (standalone VJP) it is computed into the scratch
   const bool fresh = grad_u == nullptr;
   a->ctx->launches += a->eng->kernels_per_vjp(fresh);
-  return a->eng->vjp(a->ctx->cfg, u, fresh ? a->gwork : grad_u, fresh, w, out, X, x0, Y, x1, b, c, a->xy, a->qdir,
-                     a->ctx->stream);
+  return a->eng->vjp(a->ctx->cfg, u, fresh ? a->gwork : grad_u, fresh, w, out, X, x0, Y, x1, b, c,
+                     a->xy, a->qdir, a->ctx->stream);
 }
 
 cudaError_t objective(dgsem_adjoint* a, const double* u, double* grad) {
@@ -389,7 +389,7 @@ dgsem_status dgsem_adjoint_create(dgsem_ctx* ctx, int nsteps, int checkpoint_eve
   if (a->work) a->lam = adj_alloc(a, a->len, &err);
   if (a->lam) a->lam2 = adj_alloc(a, a->len, &err);
   if (a->lam2) a->lam1 = adj_alloc(a, a->len, &err);
-  a->glen = ns ? nodes * 8 : 0;
+  a->glen = ns ? nodes * 4 : 0;
   if (a->lam1 && ns) a->gseg = adj_alloc(a, (size_t)a->every * 3 * a->glen, &err);
   if (a->gseg) a->gwork = adj_alloc(a, a->glen, &err);
   if (a->lam1 && (!ns || a->gwork)) a->xy = adj_alloc(a, ns ? (size_t)nodes * 8 : 1, &err);

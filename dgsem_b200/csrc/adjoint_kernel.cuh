@@ -35,7 +35,7 @@ template <int N>
 struct AdjArgs {
   const double* u;     // state at which the Jacobian is taken
   const double* w;     // cotangent input
-  const double* grad;  // forward BR1 gradient of u [E][4][2][ND] (Navier-Stokes)
+  const double* grad;  // Navier-Stokes: forward velocity gradient of u [E][2][2][ND]
   double* xy;          // Navier-Stokes: X~, Y~ per node [E][4][2][ND]
   double* qdir;        // Navier-Stokes: direct velocity cotangents [E][2][ND]
   double* out;         // x0 X + x1 Y + b w + c VJP (may alias X)
@@ -272,15 +272,15 @@ __global__ void __launch_bounds__(EPB* N* N) adj_viscous_kernel(const AdjArgs<N>
 #pragma unroll
   for (int v = 0; v < 4; ++v) u[v] = __ldg(p.u + ((int64_t)e * 4 + v) * ND + node);
   ns_gradient_variables(u, p.gamma, q);
-  double gx[4], gy[4];
+  double gx[2], gy[2];  // d v_c / dx, d v_c / dy
 #pragma unroll
-  for (int v = 0; v < 4; ++v) {
-    gx[v] = __ldg(p.grad + (((int64_t)e * 4 + v) * 2 + 0) * ND + node);
-    gy[v] = __ldg(p.grad + (((int64_t)e * 4 + v) * 2 + 1) * ND + node);
+  for (int v = 0; v < 2; ++v) {
+    gx[v] = __ldg(p.grad + (((int64_t)e * 2 + v) * 2 + 0) * ND + node);
+    gy[v] = __ldg(p.grad + (((int64_t)e * 2 + v) * 2 + 1) * ND + node);
   }
-  const double tau11 = (4.0 * gx[1] - 2.0 * gy[2]) * (1.0 / 3.0);
-  const double tau22 = (4.0 * gy[2] - 2.0 * gx[1]) * (1.0 / 3.0);
-  const double tau12 = gy[1] + gx[2];
+  const double tau11 = (4.0 * gx[0] - 2.0 * gy[1]) * (1.0 / 3.0);
+  const double tau22 = (4.0 * gy[1] - 2.0 * gx[0]) * (1.0 / 3.0);
+  const double tau12 = gy[0] + gx[1];
   const double t11b = sx[1] + sx[3] * q[1];
   const double t12b = sx[2] + sx[3] * q[2] + sy[1] + sy[3] * q[1];
   const double t22b = sy[2] + sy[3] * q[2];

@@ -46,7 +46,7 @@ template <int N>
 struct ViscArgs {
   const double* u;
   double* visc;  // [E][DIM][DIM + 1][ND] (may be null)
-  double* grad;  // adjoint (2D): velocity gradient [E][4][2][ND], rows 1, 2 (may be null)
+  double* grad;  // adjoint (2D): velocity gradient [E][2][2][ND] (may be null)
   int nelem;
   double gamma, mu, kappa;
   DeviceTables tab;
@@ -233,7 +233,7 @@ __device__ __forceinline__ void viscous_flux_body(const ViscArgs<N>& p) {
         for (int v = 0; v < 2; ++v)
 #pragma unroll
           for (int c = 0; c < 2; ++c)
-            p.grad[(((int64_t)e * 4 + 1 + v) * 2 + c) * ND + node] = g[c][v];
+            p.grad[(((int64_t)e * 2 + v) * 2 + c) * ND + node] = g[c][v];
       }
     }
     if (!p.visc) continue;
