@@ -794,11 +794,11 @@ dgsem_status dgsem_launch_count(const dgsem_ctx* ctx, int64_t* count) {
 }  // extern "C"
 
 // ---------------------------------------------------------------------------
-// Launch-shape autotuner: every engine has kNumVariants launch shapes of the
-// same kernel (bitwise-identical results).  Tuning times each on the real mesh
-// and state; choices are cached per (scheme, degree, element count) for the
-// process and, if DGSEM_TUNING_FILE names a file, persisted there as lines
-// "key variant".
+// Launch-shape autotuner: every engine has up to kNumVariants launch shapes of
+// the same right-hand side (0-2 with the same bits, the others to rounding).
+// Tuning times each on the real mesh and state; choices are cached per (kernel
+// revision, scheme, degree, element count) for the process and, if
+// DGSEM_TUNING_FILE names a file, persisted there as lines "key variant".
 // ---------------------------------------------------------------------------
 namespace dgsem {
 namespace tune_detail {
@@ -834,9 +834,14 @@ void tune_store(const std::string& key, int v) {
 
 }  // namespace tune_detail
 
+// Part of every key.  Raised with a change that makes another shape the fastest
+// somewhere or gives a shape number another kernel, so that choices persisted
+// with earlier kernels are timed again: 2 = shapes 0-2 are the line sweeps.
+constexpr int kTuneRevision = 2;
+
 std::string tune_key(int ndims, int n, int vf, int sf, int hg, int ns, int64_t nelem) {
   std::ostringstream k;
-  k << "d" << ndims << "_n" << n << "_vf" << vf << "_sf" << sf << "_hg" << hg << "_ns" << ns
+  k << "r" << kTuneRevision << "_d" << ndims << "_n" << n << "_vf" << vf << "_sf" << sf << "_hg" << hg << "_ns" << ns
     << "_e" << nelem;
   return k.str();
 }

@@ -317,8 +317,8 @@ dgsem_status dgsem_check_finite(dgsem_ctx* ctx);
  * runs; with the environment variable DGSEM_AUTOTUNE_WARM set, steps are
  * timed back to back instead (L2-resident small meshes).  Choices are cached
  * per (scheme, degree, element count, timing mode) for the process and, when
- * the environment variable DGSEM_TUNING_FILE names a file, persisted there.
- * Synchronous. */
+ * the environment variable DGSEM_TUNING_FILE names a file, persisted there;
+ * choices persisted with earlier kernels are not used.  Synchronous. */
 dgsem_status dgsem_autotune(dgsem_ctx* ctx, const double* u, int* chosen,
                             double* times_ms);
 /* Selects a launch shape; DGSEM_ERR_INVALID_ARG if the scheme lacks it. */
