@@ -96,25 +96,21 @@ def measured_peak():
         return 6650.0, "fallback"
 
 
-# stage kernel launched by each launch shape (dgsem_autotune / --variant)
-VARIANT_KERNELS = {
-    0: "stage_line_kernel", 1: "stage_line_kernel", 2: "stage_line_kernel",
-    3: "stage_node_kernel", 4: "stage_node_kernel", 5: "stage_pipe_kernel",
-    6: "stage_node2_kernel",
-}
+# the stage kernels (StructuredSolver.kernel_name())
 KERNEL_DESCRIPTIONS = {
-    "stage_line_kernel": "stage_line_kernel / stage_split_kernel (line sweeps, fused RHS + SSPRK3 stage)",
-    "stage_node_kernel": "stage_node_kernel (node-parallel fused RHS + SSPRK3 stage)",
-    "stage_pipe_kernel": "stage_pipe_kernel (persistent node-parallel, TMA tile streaming)",
-    "stage_node2_kernel": "stage_node2_kernel (node-parallel, two nodes per thread)",
+    "stage_split_kernel": "stage_split_kernel (line shapes, a block per group of elements)",
+    "stage_line_kernel": "stage_line_kernel (line shapes, a warp per group of elements)",
+    "stage_node_kernel": "stage_node_kernel (one thread per node)",
+    "stage_pipe_kernel": "stage_pipe_kernel (one thread per node, persistent, TMA tile streaming)",
+    "stage_node2_kernel": "stage_node2_kernel (two nodes per thread)",
 }
 
 
 def profile_value(workload: str, kernel: str, key: str):
-    """A figure of the stage kernel's committed ncu summary (profiles/), e.g.
-    traffic_bytes_per_launch (DRAM read + write bytes of one launch) or
-    fp64_flops_per_dof (FP64 add + mul + 2 x fma thread operations per DOF
-    and stage)."""
+    """A figure of the committed ncu summary (profiles/) of this kernel on this
+    workload, e.g. traffic_bytes_per_launch (DRAM read + write bytes of one
+    launch) or fp64_flops_per_dof (FP64 add + mul + 2 x fma thread operations
+    per DOF and stage); None where the kernel has no summary."""
     path = os.path.join(ROOT, "profiles", f"{kernel}_{workload}.md")
     try:
         with open(path) as f:
@@ -124,10 +120,6 @@ def profile_value(workload: str, kernel: str, key: str):
     except (OSError, ValueError):
         pass
     return None
-
-
-def profile_traffic(workload: str, kernel: str = "stage_line_kernel"):
-    return profile_value(workload, kernel, "traffic_bytes_per_launch")
 
 
 def fp64_peak(stream) -> dict:
@@ -609,8 +601,8 @@ def run_device_arm(args):
     mean_stage_s = sum(step_ms) / (3 * args.steps) * 1e-3
     achieved = dofs * bpd / mean_stage_s / 1e9
     peak, peak_kind = measured_peak()
-    kernel = VARIANT_KERNELS.get(variant, "stage_line_kernel")
-    traffic = profile_traffic(name, kernel)
+    kernel = solver.kernel_name()
+    traffic = profile_value(name, kernel, "traffic_bytes_per_launch")
     # FP64 bound: FP64 operations per launch (ncu op counters of the committed
     # summary, per DOF) over the same average launch time, against the FP64
     # FMA peak measured live on this GPU
@@ -830,6 +822,12 @@ def measure_batched(args, rank: int = 0, world: int = 1):
     mode = min(mode_ms, key=mode_ms.get)
     step_ms, launches, clocks, g = modes[mode]
     batch.set_persistent(mode == "persistent")
+    # the committed traffic figure is that of the 256 meshes with one kernel in
+    # every degree group
+    kernels = [batch.kernel_name(k) for k in range(len({N for _, N, _, _ in specs}))]
+    traffic = None
+    if mode == "per_degree" and not shard and len(set(kernels)) == 1:
+        traffic = profile_value("batched", kernels[0], "traffic_bytes_per_stage")
     # the job's time is the slowest rank's (max over ranks)
     total_ms = max_over_ranks(sum(step_ms), world, dev)
     if shard:
@@ -887,15 +885,14 @@ def measure_batched(args, rank: int = 0, world: int = 1):
                         if world > 1 else "single"),
         "vs_baseline": None, "dtype": "f64", "data": "synthetic (seeded isentropic vortices)",
         "config": batched_config(),
-        "launch_variants": variants,
+        "launch_variants": variants, "launch_kernels": kernels,
         "speedup_vs_per_instance": plain_ms / batched_ms,
         "launch_mode": mode,
         "ms_per_step_by_mode": mode_ms,
         "per_instance_ms_per_step_sum": plain_ms,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak,
-                     "traffic": profile_value("batched", "stage_node_kernel",
-                                              "traffic_bytes_per_stage"),
+                     "traffic": traffic,
                      "peak_source": f"{peak_kind} MEASURED_PEAKS.json hbm_gbs"},
         "e2e": {"value": e2e_dofs * 3 / (e2e_ms * 1e-3), "unit": "DOF-updates/s",
                 "h2d_bytes_per_step": dofs * 32, "d2h_bytes_per_step": dofs * 32},

@@ -53,6 +53,7 @@ EXPORTED = [
     "dgsem_checkpoint_write", "dgsem_checkpoint_read", "dgsem_checkpoint_write_host",
     "dgsem_checkpoint_read_host", "dgsem_set_diagnostics", "dgsem_diagnostics",
     "dgsem_geometry_from_coordinates", "dgsem_batch_set_persistent",
+    "dgsem_launch_kernel_name", "dgsem_batch_launch_kernel_name",
 ]
 
 
@@ -131,6 +132,10 @@ def lib() -> ctypes.CDLL:
     L.dgsem_batch_launch_count.argtypes = [vp, c.POINTER(c.c_int64)]
     L.dgsem_autotune.argtypes = [vp, dp, c.POINTER(c.c_int), c.POINTER(c.c_double)]
     L.dgsem_set_launch_variant.argtypes = [vp, c.c_int]
+    L.dgsem_launch_kernel_name.argtypes = [vp]
+    L.dgsem_launch_kernel_name.restype = c.c_char_p
+    L.dgsem_batch_launch_kernel_name.argtypes = [vp, c.c_int]
+    L.dgsem_batch_launch_kernel_name.restype = c.c_char_p
     L.dgsem_batch_autotune.argtypes = [vp, dp, c.POINTER(c.c_double), c.POINTER(c.c_int)]
     L.dgsem_batch_set_launch_variant.argtypes = [vp, c.c_int]
     L.dgsem_ssprk3_step_static_scratch.argtypes = [vp, dp, c.c_double, c.c_double]
@@ -159,7 +164,7 @@ def lib() -> ctypes.CDLL:
     L.dgsem_batch_set_persistent.argtypes = [vp, c.c_int]
     for name in EXPORTED:
         f = getattr(L, name)
-        if name != "dgsem_status_string":
+        if not name.endswith(("_status_string", "_kernel_name")):
             f.restype = ctypes.c_int
     _lib = L
     return L

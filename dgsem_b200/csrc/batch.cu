@@ -312,6 +312,13 @@ dgsem_status dgsem_batch_set_launch_variant(dgsem_batch* b, int variant) {
   return DGSEM_OK;
 }
 
+const char* dgsem_batch_launch_kernel_name(const dgsem_batch* b, int group) {
+  if (!b || group < 0 || group >= (int)b->groups.size()) return nullptr;
+  // batched launches of shapes 5 and 6 run shape 3's kernel
+  const EngineBase& e = *b->groups[group].engine;
+  return e.variant() >= 3 ? "stage_node_kernel" : e.kernel_name();
+}
+
 dgsem_status dgsem_batch_create(const dgsem_mesh_desc* meshes, int n_meshes,
                                 const dgsem_scheme_desc* scheme, void* stream,
                                 dgsem_batch** out) {

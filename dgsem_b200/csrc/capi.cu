@@ -910,6 +910,10 @@ dgsem_status dgsem_set_launch_variant(dgsem_ctx* ctx, int variant) {
   return DGSEM_OK;
 }
 
+const char* dgsem_launch_kernel_name(const dgsem_ctx* ctx) {
+  return ctx ? ctx->engine->kernel_name() : nullptr;
+}
+
 dgsem_status dgsem_autotune(dgsem_ctx* ctx, const double* u, int* chosen, double* times_ms) {
   using namespace dgsem::tune_detail;
   if (!ctx || !u) return DGSEM_ERR_INVALID_ARG;

@@ -93,6 +93,8 @@ class EngineBase {
   // depends on it
   virtual void set_mesh_size(int64_t nelem) = 0;
   virtual int num_variants() const = 0;
+  // stage kernel that the current launch shape runs
+  virtual const char* kernel_name() const = 0;
 };
 
 std::unique_ptr<EngineBase> make_engine(int ndims, int n, int vf, int sf,
@@ -513,6 +515,12 @@ class Engine final : public EngineBase {
     load_variant(variant_);
   }
   int variant() const override { return variant_; }
+  const char* kernel_name() const override {
+    if (kNode2 && variant_ == 6) return "stage_node2_kernel";
+    if (kPipe && variant_ == 5) return "stage_pipe_kernel";
+    if (variant_ >= 3) return "stage_node_kernel";
+    return use_split() ? "stage_split_kernel" : "stage_line_kernel";
+  }
   // shapes 5 and 6 exist for single-mesh launches; batched launches run them as 3
   int num_variants() const override { return kNode2 ? 7 : kPipe ? 6 : kNode ? 5 : 3; }
 

@@ -373,6 +373,10 @@ class StructuredSolver:
         C.check(C.lib().dgsem_set_launch_variant(self._ctx, int(variant)),
                 "dgsem_set_launch_variant")
 
+    def kernel_name(self) -> str:
+        """Stage kernel that the current launch shape runs (dgsem_launch_kernel_name)."""
+        return C.lib().dgsem_launch_kernel_name(self._ctx).decode()
+
     def launch_count(self) -> int:
         c = ctypes.c_int64()
         C.check(C.lib().dgsem_launch_count(self._ctx, ctypes.byref(c)), "dgsem_launch_count")
@@ -637,6 +641,13 @@ class BatchSolver:
         """One launch shape for every degree group (dgsem_batch_set_launch_variant)."""
         C.check(C.lib().dgsem_batch_set_launch_variant(self._h, int(variant)),
                 "dgsem_batch_set_launch_variant")
+
+    def kernel_name(self, group: int) -> str:
+        """Stage kernel of a degree group (dgsem_batch_launch_kernel_name)."""
+        name = C.lib().dgsem_batch_launch_kernel_name(self._h, int(group))
+        if name is None:
+            raise IndexError(group)
+        return name.decode()
 
     def set_persistent(self, enable: bool = True) -> None:
         """One persistent launch per stage over all meshes (dgsem_batch_set_persistent)."""

@@ -268,6 +268,9 @@ dgsem_status dgsem_batch_launch_count(const dgsem_batch* b, int64_t* count);
  * degree group of the batch, as dgsem_batch_autotune would after timing;
  * DGSEM_ERR_INVALID_ARG if a group's scheme lacks it. */
 dgsem_status dgsem_batch_set_launch_variant(dgsem_batch* b, int variant);
+/* Name of the stage kernel of the per-degree launches of degree group `group`
+ * (distinct degrees, ascending); NULL if there is no such group. */
+const char* dgsem_batch_launch_kernel_name(const dgsem_batch* b, int group);
 dgsem_status dgsem_batch_set_persistent(dgsem_batch* b, int enable);
 
 /* Hennemann-Gassner blending factor per element and troubled-cell flag
@@ -323,6 +326,10 @@ dgsem_status dgsem_autotune(dgsem_ctx* ctx, const double* u, int* chosen,
                             double* times_ms);
 /* Selects a launch shape; DGSEM_ERR_INVALID_ARG if the scheme lacks it. */
 dgsem_status dgsem_set_launch_variant(dgsem_ctx* ctx, int variant);
+/* Name of the stage kernel that the current launch shape runs on this mesh
+ * (stage_split_kernel, stage_line_kernel, stage_node_kernel, stage_pipe_kernel
+ * or stage_node2_kernel); NULL for a NULL context. */
+const char* dgsem_launch_kernel_name(const dgsem_ctx* ctx);
 
 /* Fused per-step diagnostics (replaces the reference's AnalysisObserver with
  * VolumeAverageEuler, observer/analysis_observer.hpp:56-110,

@@ -143,3 +143,8 @@ def test_product_has_no_cpu_path(monkeypatch, tmp_path):
     monkeypatch.setattr(C, "_lib", None)
     with pytest.raises(FileNotFoundError):
         C.lib()
+
+
+def test_kernel_name_without_a_context():
+    assert C.lib().dgsem_launch_kernel_name(None) is None
+    assert C.lib().dgsem_batch_launch_kernel_name(None, 0) is None
