@@ -672,7 +672,9 @@ class Scheme:
     shock_capturing: bool = False
     alpha_max: float = 0.5
     alpha_min: float = 0.001
-    bc: str = "periodic"            # "periodic" | "dmr"
+    bc: str = "periodic"            # "periodic" | "dmr" | "walls"
+    # bc "walls" (2D Navier-Stokes): per face None (periodic), "noslip" or "slip"
+    walls: tuple = (None, None, None, None)
     viscous: bool = False
     mu: float = 0.0
     prandtl: float = 0.72
@@ -867,6 +869,30 @@ def _volume_fv_2d(s: Scheme, U, scale):
     return du
 
 
+def _volume_fv_3d(s: Scheme, U, scale):
+    """volume_flux.hpp:513-630 FV subcell integral (3D) with LLF on the subcell
+    normals of global_def.hpp:296-440: Ja^dir of the line's first node plus the
+    running sums of w_f sum_m D(f, m) Ja^dir(m)."""
+    n = s.n
+    iw, w, D = s.basis.inv_weights, s.basis.weights, s.basis.D
+    JA = _grid(s, s.geo.ja)
+    du = np.zeros_like(U)
+    for d, ax in enumerate((-2, -3, -4)):  # node axis of direction d before var
+        u = np.moveaxis(U, ax, 0)
+        ja = np.moveaxis(JA[..., d, :], ax, 0)
+        out = np.moveaxis(du, ax, 0)
+        nrm = ja[0]
+        for f in range(1, n):
+            for m in range(n):
+                nrm = nrm + (w[f - 1] * D[f - 1, m]) * ja[m]
+            fs = np.moveaxis(flux_llf(np.moveaxis(u[f - 1], -1, 0), np.moveaxis(u[f], -1, 0),
+                                      np.moveaxis(nrm, -1, 0), s.gamma), 0, -1)
+            sc = scale[..., None, None, None]
+            out[f - 1] += (sc * iw[f - 1]) * fs
+            out[f] -= (sc * iw[f]) * fs
+    return du
+
+
 def dmr_state(x, y, t, gamma):
     """Double Mach reflection state (examples/Euler2D/double_mach_reflection/
     double_mach_reflection_structured.cpp:9-32)."""
@@ -922,6 +948,13 @@ def _surface_fluxes(s: Scheme, U, t):
         SF[:, :, 3] = np.roll(fy, -1, axis=1)
         if s.bc == "dmr":
             _dmr_boundary(s, U, JA, SF, t)
+        for face, kind in _wall_faces(s):
+            el, d, side = _face_slices(s, face)
+            ui, nrm = U[el], JA[el][..., d, :]
+            uw = _reflected(ui, nrm)
+            a, b = (ui, uw) if side else (uw, ui)
+            SF[el[:2] + (face,)] = np.moveaxis(
+                sf(np.moveaxis(a, -1, 0), np.moveaxis(b, -1, 0), np.moveaxis(nrm, -1, 0), g), 0, -1)
         return SF
     nx, ny, nz = cells
     SF = np.zeros((nx, ny, nz, 6, n, n, nv))
@@ -936,6 +969,31 @@ def _surface_fluxes(s: Scheme, U, t):
         SF[:, :, :, 2 * d] = fl
         SF[:, :, :, 2 * d + 1] = np.roll(fl, -1, axis=ax_e)
     return SF
+
+
+def _wall_faces(s: Scheme):
+    """(face, kind) of the wall faces."""
+    return [(f, k) for f, k in enumerate(s.walls) if k] if s.bc == "walls" else []
+
+
+def _face_slices(s: Scheme, face):
+    """Index of the boundary face's nodes in [ie, je, jn, in, ..] arrays, its
+    direction and side."""
+    d, side = divmod(face, 2)
+    e, m = (-1, s.n - 1) if side else (0, 0)
+    full = slice(None)
+    return ((e, full, full, m) if d == 0 else (full, e, m, full)), d, side
+
+
+def _reflected(ui, nrm):
+    """MixedDirichletSlipWallBC::reflect_state (dirichlet_boundary.hpp:207-220)."""
+    rho = ui[..., 0]
+    vx = ui[..., 1] / rho
+    vy = ui[..., 2] / rho
+    nn2 = nrm[..., 0] * nrm[..., 0] + nrm[..., 1] * nrm[..., 1]
+    vn = (vx * nrm[..., 0] + vy * nrm[..., 1]) / nn2
+    return np.stack([rho, rho * (vx - 2.0 * vn * nrm[..., 0]), rho * (vy - 2.0 * vn * nrm[..., 1]),
+                     ui[..., 3]], -1)
 
 
 def _dmr_boundary(s: Scheme, U, JA, SF, t):
@@ -967,12 +1025,7 @@ def _dmr_boundary(s: Scheme, U, JA, SF, t):
     c = C[:, 0, 0, :, :]
     nrm = JA[:, 0, 0, :, 1, :]
     uo = np.moveaxis(dmr_state(c[..., 0], c[..., 1], t, g), 0, -1)
-    rho = ui[..., 0]
-    vx = ui[..., 1] / rho
-    vy = ui[..., 2] / rho
-    nn2 = nrm[..., 0] * nrm[..., 0] + nrm[..., 1] * nrm[..., 1]
-    vn = (vx * nrm[..., 0] + vy * nrm[..., 1]) / nn2
-    uw = np.stack([rho, rho * (vx - 2.0 * vn * nrm[..., 0]), rho * (vy - 2.0 * vn * nrm[..., 1]), ui[..., 3]], -1)
+    uw = _reflected(ui, nrm)
     use_d = (c[..., 0] < 1.0 / 6.0)[..., None]
     SF[:, 0, 2] = np.where(use_d, flux(uo, ui, nrm), flux(uw, ui, nrm))
     # face 3 (top): Dirichlet, flux(inner, outer)
@@ -1012,8 +1065,9 @@ def gradient_variables(U, gamma):
 
 
 def br1_gradient(s: Scheme, U):
-    """BR1 lifted gradient, 2D periodic (structured_solver.hpp:437-452;
-    parabolic_gradient.hpp:480-818).  Returns grad[.., jn, in, var, dim]."""
+    """BR1 lifted gradient, 2D, periodic or with adiabatic walls
+    (structured_solver.hpp:437-452; parabolic_gradient.hpp:480-818).  Returns
+    grad[.., jn, in, var, dim]."""
     n = s.n
     Dh = s.basis.Dhat
     JA = _grid(s, s.geo.ja)
@@ -1037,6 +1091,19 @@ def br1_gradient(s: Scheme, U):
     qy = 0.5 * (np.roll(q, 1, axis=1)[:, :, n - 1, :, :] + q[:, :, 0, :, :])   # face 2
     qx_r = np.roll(qx, -1, axis=0)
     qy_t = np.roll(qy, -1, axis=1)
+    # wall faces: q^ = q of the wall (navier_stokes_wall_boundary.hpp:82-99
+    # no-slip: velocity zero; :162-190 slip: the normal velocity removed)
+    for face, kind in _wall_faces(s):
+        el, d, side = _face_slices(s, face)
+        qw = q[el].copy()
+        if kind == "noslip":
+            qw[..., 1:3] = 0.0
+        else:
+            nrm = JA[el][..., d, :]
+            vn = ((qw[..., 1] * nrm[..., 0] + qw[..., 2] * nrm[..., 1])
+                  / (nrm[..., 0] ** 2 + nrm[..., 1] ** 2))
+            qw[..., 1:3] -= vn[..., None] * nrm
+        (qx, qx_r, qy, qy_t)[face][el[:2]] = qw
     lL = s.basis.lhat_left[0]
     lR = s.basis.lhat_right[n - 1]
     # :689-782 lifting with the element's own face normals
@@ -1091,7 +1158,73 @@ def viscous_terms(s: Scheme, U, grad):
     SF[:, :, 1] = np.roll(fx_face, -1, axis=0)
     SF[:, :, 2] = fy_face
     SF[:, :, 3] = np.roll(fy_face, -1, axis=1)
+    # wall faces: the inner -F_v . n on the momentum at no-slip walls
+    # (navier_stokes_wall_boundary.hpp:101-131), nothing at slip walls
+    for face, kind in _wall_faces(s):
+        el, d, side = _face_slices(s, face)
+        fw = np.zeros_like(U[el])
+        if kind == "noslip":
+            nrm = JA[el][..., d, :]
+            fv = Fv[el][..., 0] * nrm[..., 0, None] + Fv[el][..., 1] * nrm[..., 1, None]
+            fw[..., 1:3] = fv[..., 1:3]
+        SF[el[:2] + (face,)] = fw
     _surface_integral(s, du, SF)
+    return du
+
+
+def viscous_rhs_3d(s: Scheme, U):
+    """Viscous terms on 3D periodic boxes: BR1 gradient of (v, T)
+    (parabolic_gradient.hpp:17-437), -F_v (compressible_navier_stokes3D.hpp:
+    72-124), weak-form divergence with the one-sided interface flux
+    (parabolic_viscous.hpp, 3D functors), before the shared -1/J scaling."""
+    n, g = s.n, s.gamma
+    Dh = s.basis.Dhat
+    lL, lR = s.basis.lhat_left[0], s.basis.lhat_right[n - 1]
+    JA, IJ = _grid(s, s.geo.ja), _grid(s, s.geo.inv_j)
+    rho = U[..., 0]
+    v = [U[..., 1 + d] / rho for d in range(3)]
+    p = (g - 1.0) * (U[..., 4] - 0.5 * (U[..., 1] * v[0] + U[..., 2] * v[1] + U[..., 3] * v[2]))
+    q = np.stack(v + [p / rho], axis=-1)
+
+    def line_product(d, a):
+        """sum_i Dhat(m, i) a_i along direction d of [.., kn, jn, in, x]."""
+        return np.moveaxis(np.tensordot(Dh, a, axes=(1, a.ndim - 2 - d)), 0, a.ndim - 2 - d)
+
+    def node(d, m):
+        """Index of the nodes at position m of the lines along d."""
+        return (Ellipsis,) + tuple(m if ax == d else slice(None) for ax in (2, 1, 0)) + (slice(None),)
+
+    grad = np.zeros(q.shape + (3,))
+    for d in range(3):
+        dq = line_product(d, q)
+        lo = 0.5 * (np.roll(q, 1, axis=d)[node(d, n - 1)] + q[node(d, 0)])
+        hi = np.roll(lo, -1, axis=d)
+        dq[node(d, 0)] -= lL * lo
+        dq[node(d, n - 1)] += lR * hi
+        # the metric terms of the face nodes are the nodes' own: one transform
+        # for the volume and the lifted part
+        grad += dq[..., None] * JA[..., d, :][..., None, :]
+    grad *= IJ[..., None, None]
+    kappa = g / ((g - 1.0) * s.prandtl)
+    div = grad[..., 0, 0] + grad[..., 1, 1] + grad[..., 2, 2]
+    F = np.zeros(U.shape + (3,))  # -F_v
+    for c in range(3):
+        energy = kappa * grad[..., 3, c]
+        for r in range(3):
+            tau = grad[..., r, c] + grad[..., c, r]
+            if r == c:
+                tau = tau - 2.0 / 3.0 * div
+            energy = energy + v[r] * tau
+            F[..., 1 + r, c] = -s.mu * tau
+        F[..., 4, c] = -s.mu * energy
+    du = np.zeros_like(U)
+    for d in range(3):
+        f = np.sum(F * JA[..., d, :][..., None, :], axis=-1)
+        lo = f[node(d, 0)]  # the high-side element's own flux at its low face
+        part = line_product(d, f)
+        part[node(d, 0)] -= lL * lo
+        part[node(d, n - 1)] += lR * np.roll(lo, -1, axis=d)
+        du += part
     return du
 
 
@@ -1107,15 +1240,16 @@ def rhs(s: Scheme, u, t=0.0, return_alpha=False):
         bshape = alpha.shape + (1,) * nd
         scale_dg = np.where(flagged, 1.0 - alpha, 1.0).reshape(bshape)
         du = _volume_split(s, U, JA, scale_dg)
-        if nd != 2:
-            raise NotImplementedError("FV subcell integral is restated for 2D")
-        du = du + _volume_fv_2d(s, U, np.where(flagged, alpha, 0.0))
+        volume_fv = _volume_fv_2d if nd == 2 else _volume_fv_3d
+        du = du + volume_fv(s, U, np.where(flagged, alpha, 0.0))
     else:
         du = _volume_split(s, U, JA, 1.0)
     SF = _surface_fluxes(s, U, t)
     if s.viscous:
-        grad = br1_gradient(s, U)
-        du = du + viscous_terms(s, U, grad)
+        if nd == 2:
+            du = du + viscous_terms(s, U, br1_gradient(s, U))
+        else:
+            du = du + viscous_rhs_3d(s, U)
     _surface_integral(s, du, SF)
     du = du * (-_grid(s, s.geo.inv_j))[..., None]
     out = du.reshape(np.asarray(u).shape)

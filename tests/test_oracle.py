@@ -245,3 +245,118 @@ def test_kennedy_gruber_known_answer(nd):
     if nd == 2:
         assert _kg_exact(primL, primR, normal, gamma) == [
             F(-9, 128), F(15, 16), F(-187, 1024), F(-1965, 8192)]
+
+
+# ---- the oracle's 3D shock capturing, 3D viscous terms and walls -----------
+def _extruded(s2, s3, axes, u2):
+    """The 2D state u2 (reference layout) on the 3D mesh, constant along the
+    third axis; axes = (axis of x, axis of y) in 3D."""
+    n = s2.n
+    rest = ({0, 1, 2} - set(axes)).pop()
+    U2 = u2.reshape(s2.cells + (n, n, 4))  # [ie, je, jn, in]
+    u3 = np.zeros(s3.cells + (n,) * 3 + (5,))  # [.., kn, jn, in, var]
+    rows = [0, 1 + axes[0], 1 + axes[1], 4]
+    src = U2 if axes[0] < axes[1] else np.swapaxes(np.swapaxes(U2, 0, 1), 2, 3)
+    src = np.expand_dims(np.expand_dims(src, rest), 3 + 2 - rest)
+    u3[..., rows] = np.broadcast_to(src, u3.shape[:-1] + (4,))
+    return u3.reshape(s3.cells + (n ** 3, 5))
+
+
+@pytest.mark.parametrize("axes", [(0, 1), (1, 2), (2, 0)])
+@pytest.mark.parametrize("part", ["viscous", "fv"])
+def test_oracle_3d_reduces_to_2d(part, axes):
+    """On a state that does not depend on one axis and does not move along it, the
+    3D viscous terms and the 3D FV subcell integral are the 2D ones (which the
+    fixtures from the compiled reference pin)."""
+    n, cells2 = 4, (3, 4)
+    left2, right2 = (0.0, 0.0), (2.0, 3.0)
+    s2 = do.Scheme(ndims=2, polydeg=n - 1, cells=cells2, left=left2, right=right2, viscous=True,
+                   mu=0.02)
+    rest = ({0, 1, 2} - set(axes)).pop()
+    cells3, right3 = [0, 0, 0], [0.0] * 3
+    for a, ax in enumerate(axes):
+        cells3[ax], right3[ax] = cells2[a], right2[a]
+    cells3[rest], right3[rest] = 2, 1.7
+    s3 = do.Scheme(ndims=3, polydeg=n - 1, cells=tuple(cells3), left=(0.0,) * 3, right=tuple(right3),
+                   viscous=True, mu=0.02)
+    rng = np.random.default_rng(5)
+    u2 = np.empty(cells2 + (n * n, 4))
+    u2[..., 0] = rng.uniform(1.0, 2.0, u2.shape[:-1])
+    u2[..., 1:3] = rng.standard_normal(u2.shape[:-1] + (2,))
+    u2[..., 3] = 12.0 + rng.uniform(0.0, 2.0, u2.shape[:-1])
+    u3 = _extruded(s2, s3, axes, u2)
+    U2, U3 = do._grid(s2, u2), do._grid(s3, u3)
+    if part == "viscous":
+        d2 = do.viscous_terms(s2, U2, do.br1_gradient(s2, U2))
+        d3 = do.viscous_rhs_3d(s3, U3)
+    else:
+        a2 = rng.uniform(0.0, 0.5, cells2)
+        a3 = np.expand_dims(a2 if axes[0] < axes[1] else a2.T, rest)
+        d2 = do._volume_fv_2d(s2, U2, a2)
+        d3 = do._volume_fv_3d(s3, U3, np.broadcast_to(a3, s3.cells))
+    d2 = d2 * do._grid(s2, s2.geo.inv_j)[..., None]
+    d3 = d3 * do._grid(s3, s3.geo.inv_j)[..., None]
+    want = _extruded(s2, s3, axes, d2.reshape(u2.shape))
+    # the pressure along the third axis (whose end fluxes the surface term
+    # balances) is in that axis' momentum only
+    diff = np.abs(np.delete(d3.reshape(u3.shape) - want, 1 + rest, axis=-1))
+    assert np.max(diff) <= 1e-12 * np.max(np.abs(want)), np.max(diff)
+
+
+def test_oracle_slip_walls_mirror_symmetry():
+    """Without viscosity a slip-wall box is a quarter of the mirrored periodic
+    box; with it the gradient at the walls still is."""
+    n, cells = 4, (3, 2)
+    kw = dict(ndims=2, polydeg=n - 1, left=(0.0, 0.0))
+    sw = do.Scheme(cells=cells, right=(1.5, 1.0), bc="walls", periodic=False,
+                   walls=("slip",) * 4, **kw)
+    sp = do.Scheme(cells=(6, 4), right=(3.0, 2.0), **kw)
+    rng = np.random.default_rng(9)
+    u = np.empty(cells + (n * n, 4))
+    u[..., 0] = rng.uniform(1.0, 2.0, u.shape[:-1])
+    u[..., 1:3] = rng.standard_normal(u.shape[:-1] + (2,))
+    u[..., 3] = 12.0 + rng.uniform(0.0, 2.0, u.shape[:-1])
+    U = do._grid(sw, u)
+    sx, sy = np.array([1, -1, 1, 1.0]), np.array([1, 1, -1, 1.0])
+    right = np.concatenate([U, U[::-1, :, :, ::-1] * sx], axis=0)
+    full = np.concatenate([right, right[:, ::-1, ::-1] * sy], axis=1)
+    ref = do.rhs(sp, full.reshape(6, 4, n * n, 4))[:3, :2]
+    got = do.rhs(sw, u)
+    assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
+    g_ref = do.br1_gradient(sp, full)[:3, :2]
+    g = do.br1_gradient(sw, U)
+    assert np.max(np.abs(g - g_ref)) <= 1e-12 * np.max(np.abs(g_ref))
+
+
+def test_oracle_no_slip_wall_terms():
+    """A no-slip wall replaces the face values: q^ = (rho, 0, 0, T), and the
+    viscous flux through it is the inner one on the momentum, none on the energy."""
+    n, cells = 4, (2, 3)
+    s = do.Scheme(ndims=2, polydeg=n - 1, cells=cells, left=(0.0, 0.0), right=(1.0, 1.0),
+                  periodic=False, bc="walls", walls=(None, None, "noslip", "slip"), viscous=True,
+                  mu=0.1)
+    sp = do.Scheme(ndims=2, polydeg=n - 1, cells=cells, left=(0.0, 0.0), right=(1.0, 1.0),
+                   viscous=True, mu=0.1)
+    rng = np.random.default_rng(3)
+    u = rng.uniform(1.0, 2.0, cells + (n * n, 4)) + np.array([0, 0, 0, 4.0])
+    U = do._grid(s, u)
+    q = do.gradient_variables(U, 1.4)
+    JA, IJ = do._grid(s, s.geo.ja), do._grid(s, s.geo.inv_j)
+    lL = s.basis.lhat_left[0]
+    # gradient: the periodic one with the wall's value instead of the average
+    qp = 0.5 * (np.roll(q, 1, axis=1)[:, 0, n - 1] + q[:, 0, 0])
+    qw = q[:, 0, 0].copy()
+    qw[..., 1:3] = 0.0
+    want = do.br1_gradient(sp, U)[:, 0, 0]
+    want = want + ((-lL) * (qw - qp))[..., None] * JA[:, 0, 0, :, 1][..., None, :] * IJ[
+        :, 0, 0][..., None, None]
+    assert np.allclose(do.br1_gradient(s, U)[:, 0, 0], want, rtol=1e-13, atol=1e-13)
+    # fluxes from the same gradient: bottom face against the periodic scheme's
+    grad = do.br1_gradient(s, U)
+    d = do.viscous_terms(s, U, grad) - do.viscous_terms(sp, U, grad)
+    assert np.abs(d[:, 0, 0, :, :3]).max() <= 1e-12 * np.abs(grad).max()  # own flux both times
+    own_energy = d[:, 0, 0, :, 3] / lL
+    assert np.abs(own_energy).min() > 0.0  # the energy flux is what the wall takes away
+    # the slip wall at the top carries none at all
+    top = do.viscous_terms(s, U, grad)[:, -1, n - 1] - do.viscous_terms(sp, U, grad)[:, -1, n - 1]
+    assert np.abs(top[..., 1:]).min() > 0.0
