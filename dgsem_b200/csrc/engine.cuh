@@ -147,7 +147,7 @@ inline StageArgs<N> stage_args_common(const EngineConfig& cfg, double a, double 
 }
 
 // Line shapes (stage_line_kernel.cuh): 0 = the split or the sweep form by the
-// mesh's size (Engine::split_by_size), 1 = split, 2 = sweep with another
+// mesh's size (Engine::split_waves), 1 = split, 2 = sweep with another
 // register cap than 0's.  Resident blocks per SM requested from the register
 // allocator: the sweeps get 168 registers (12 warps per SM) where a line's
 // data fit them, 255 (8 warps) at long lines, and shape 2 128 (16 warps) at
@@ -303,25 +303,48 @@ class Engine final : public EngineBase {
       if (v == 6) attr(node2_kernel(), Node2Shape<N, VF>::smem_bytes);
   }
 
-  // Shape 0 runs the split form on meshes too small to fill the GPU with one
-  // warp per group of elements (`warps` of the sweep); both give the same
-  // bits.  us per stage on a B200, split / sweep, near the crossings:
-  //   2D n = 3   723 warps 5.7 / 7.1, 2 161: 11.0 / 10.1
-  //      n = 4  1513: 10.8 / 12.2, 3 200: 18.7 / 15.5 (64^2 elements 4.7 / 6.3)
-  //      n = 6  2290: 27.0 / 27.6, 14 259: 173 / 107
-  //      n = 8  1600: 35 / 50, 10 000: 191 / 124
-  //      shock capturing n = 4: 32: 7.1 / 13, 1 800: 21.4 / 24.8, 3 200: 25.6 /
-  //      18.1; n = 5: 960: 31 / 28, 2 731: 37 / 26
-  //   3D n = 4   108: 2.9 / 6.9, 1 372: 13.5 / 10.1
-  //      n = 5   125: 3.2 / 9.3, 1 331: 14.4 / 14.2
+  // Shape 0 runs the split form on meshes that give the sweep fewer than
+  // split_waves() waves: `nelem` / EPW warps on WPB * MINB warp slots per SM.
+  // A sweep's time is one lane's chain per wave; the split form's chain is a
+  // third of it, but its blocks fill the GPU sooner.  Both give the same bits.
+  // Measured on a B200 (1776 slots, 1184 at long lines) at 14 sizes of 0.1 to 3.3
+  // waves per form; split / sweep time at the two sizes around the crossing, the
+  // last column the crossing in waves:
+  //   2D Chandrashekar, vortex  n = 4: 0.94 at 0.95, 1.07 at 1.20    1.05
+  //                             n = 2, 3, 5-8: between 0.93 and 1.05
+  //      KH, HLLC or Ranocha, n = 4: 0.91, 0.88 at 0.70, 1.01 at 0.85  0.84
+  //      Kennedy-Gruber n = 4   0.95 at 0.50, 1.15 at 0.70           0.55
+  //      viscous n = 4, 5, 8    1.01, 0.98, 1.02 at 0.70             0.7
+  //   2D shock capturing, KH    n = 2, 3, 4: 1.02, 1.10, 1.21 at 0.85  0.65-0.8
+  //      double Mach n = 4      0.81 at 0.85, 0.98 at 2.1, 1.05 at 2.6  2.2
+  //                             n = 5: 0.92 at 0.50, 1.10 at 0.70    0.6
+  //                             n = 6, 7, 8: 0.92 at 0.20, 1.08 at 0.35  0.28
+  //      viscous n = 3, 4, 5    0.72 at 0.20, 1.12 at 0.35, 1.10 at 0.7  0.2-0.35
+  //   3D n = 2, 3, 4            0.67, 0.89, 0.74 at 0.20, 0.94, 1.13, 0.94 at
+  //                             0.35, 0.98, 1.04, 1.08 at 0.50       0.3-0.5
+  //      n = 5                  0.97 at 0.68, 1.12 at 0.84 (0.91 at 1.02, where
+  //                             the sweep starts its second wave)    0.7
+  //      shock capturing n = 2-4: 0.84 at 0.20, 1.10 at 0.35         0.28
+  //                             n = 5: 0.93 at 0.49, 1.14 at 0.68    0.55
+  //      viscous n = 2-4        0.81-1.04 at 0.20, 0.96-1.13 at 0.35  0.2-0.4
+  // Steep lines lengthen the sweep's chain, so shock capturing at n <= 4 crosses
+  // anywhere from 0.65 (smooth) to 2.2 waves (Mach 10): 0.85 loses at most a
+  // quarter at either.
   void set_mesh_size(int64_t nelem) override {
+    using L = LineLaunch<DIM, N, 0>;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int64_t warps = (nelem + LG::EPW - 1) / LG::EPW;
-    split_ = warps < split_below();
+    split_ = (double)warps < split_waves() * (sms * L::WPB * L::MINB);
     loaded_ &= ~1u;
     load_variant(variant_);
   }
-  static constexpr int64_t split_below() {
-    return DIM == 3 ? 700 : HG ? (N > 4 ? 800 : 2000) : N <= 3 ? 1400 : 2400;
+  static constexpr double split_waves() {
+    if (DIM == 3) return N == 5 ? (HG ? 0.55 : 0.7) : 0.3;
+    if (NS) return HG ? 0.3 : 0.7;
+    if (HG) return N <= 4 ? 0.85 : N == 5 ? 0.6 : 0.28;
+    return VF == VF_KENNEDY_GRUBER ? 0.55 : 0.95;
   }
 
   // node-parallel shapes: split form with shock capturing or with the

@@ -35,7 +35,7 @@ CHANNEL = (None, None, "noslip", "slip")
 BOX = ("slip", "noslip", "noslip", "slip")
 CASES = [
     # 2D, split form of the scheme
-    _case(2, 2, (187, 124), SWEEP, "ranocha"),
+    _case(2, 2, (199, 149), SWEEP, "ranocha"),
     _case(2, 3, (149, 121), SWEEP, "kennedy_gruber"),
     _case(2, 4, (151, 131), SWEEP, "ranocha"),
     _case(2, 4, (149, 133), SWEEP, "chandrashekar", "hllc"),
@@ -51,7 +51,7 @@ CASES = [
     _case(2, 4, (264, 66), SWEEP, sf="hllc", hg=True, bc="dmr"),
     _case(2, 4, (262, 66), SWEEP, hg=True, bc="dmr"),
     _case(2, 5, (10, 12), SPLIT, hg=True),
-    _case(2, 5, (83, 61), SWEEP, hg=True),
+    _case(2, 5, (97, 79), SWEEP, hg=True),
     _case(2, 8, (61, 59), SWEEP, hg=True),
     # viscous terms, with shock capturing, with walls
     _case(2, 4, (9, 7), SPLIT, viscous=True),
