@@ -194,45 +194,6 @@ __device__ __forceinline__ void diag_block_store(double* acc, double* red, doubl
   }
 }
 
-// ---------------------------------------------------------------------------
-// Element / node index helpers
-// ---------------------------------------------------------------------------
-
-template <int DIM>
-struct ElemIdx {
-  int64_t i[3];
-};
-
-template <int DIM>
-__device__ __forceinline__ ElemIdx<DIM> elem_coords(int64_t e, const int64_t* cells) {
-  ElemIdx<DIM> r;
-  r.i[0] = e % cells[0];
-  if (DIM == 2) {
-    r.i[1] = e / cells[0];
-    r.i[2] = 0;
-  } else {
-    r.i[1] = (e / cells[0]) % cells[1];
-    r.i[2] = e / (cells[0] * cells[1]);
-  }
-  return r;
-}
-
-// Element index over the axes other than c (tables.hpp other_axes_count).
-template <int DIM>
-__device__ __forceinline__ int64_t eidx_other(const ElemIdx<DIM>& ei, int c,
-                                              const int64_t* cells) {
-  if (DIM == 2) return c == 0 ? ei.i[1] : ei.i[0];
-  if (c == 0) return ei.i[1] + cells[1] * ei.i[2];
-  if (c == 1) return ei.i[0] + cells[0] * ei.i[2];
-  return ei.i[0] + cells[0] * ei.i[1];
-}
-
-template <int DIM>
-__device__ __forceinline__ int64_t elem_linear(const ElemIdx<DIM>& ei, const int64_t* cells) {
-  if (DIM == 2) return ei.i[0] + cells[0] * ei.i[1];
-  return ei.i[0] + cells[0] * (ei.i[1] + cells[1] * ei.i[2]);
-}
-
 // Node index of position m along line `line` in direction dir.
 template <int DIM, int N>
 __device__ __forceinline__ int line_node(int dir, int line, int m) {
@@ -240,12 +201,6 @@ __device__ __forceinline__ int line_node(int dir, int line, int m) {
   if (dir == 0) return m + N * line;
   if (dir == 1) return (line % N) + N * m + N * N * (line / N);
   return line + N * N * m;
-}
-
-// Node index of face node fn on the face of direction dir at position pos.
-template <int DIM, int N>
-__device__ __forceinline__ int face_node(int dir, int fn, int pos) {
-  return line_node<DIM, N>(dir, fn, pos);
 }
 
 __device__ __forceinline__ double ja_at(const double* tab, int64_t eidx, int nd,
@@ -475,14 +430,6 @@ __device__ double hg_alpha_2d(const double* us_el, int ND, const BasisConst<N>& 
 // ---------------------------------------------------------------------------
 // Shared by the stage kernels
 // ---------------------------------------------------------------------------
-// Node position in a shared-memory plane, optionally padded by one slot per N
-// nodes.  The node-parallel kernels, whose warps read 32 consecutive nodes
-// shifted along one line, use the unpadded layout (PAD = false).
-template <int N, bool PAD = true>
-__device__ __forceinline__ constexpr int padn(int node) {
-  return PAD ? node + node / N : node;
-}
-
 // Programmatic dependent launch: the stage kernels are launched with
 // programmatic stream serialization, so a stage kernel may be scheduled while
 // the previous kernel on its stream is still draining.  Each block first
@@ -496,14 +443,13 @@ __device__ __forceinline__ void stage_dependency_sync() {
 
 // The u tile [el][var][node] of a block in two steps: issue() starts every
 // global load of this thread for a full tile (ne == EPB) into registers,
-// store() writes them to the padded shared layout `us` (a partial tile is
-// loaded and stored in store()).  Work placed between the two overlaps the
-// loads' latency, and the block waits for one global round trip instead of
-// one per loop iteration.
-template <int N, int NV, int ND, int NDP, int EPB, int NT>
+// store() writes them to the shared tile `us` (a partial tile is loaded and
+// stored in store()).  Work placed between the two overlaps the loads' latency,
+// and the block waits for one global round trip instead of one per loop
+// iteration.
+template <int NV, int ND, int EPB, int NT>
 struct ElementTileLoad {
   static constexpr int TILE = EPB * NV * ND, PER = (TILE + NT - 1) / NT;
-  static constexpr bool PAD = NDP != ND;
   double v[PER];
   __device__ __forceinline__ void issue(const double* src, int ne, int tid) {
     if (ne != EPB) return;
@@ -516,23 +462,13 @@ struct ElementTileLoad {
 #pragma unroll
       for (int r = 0; r < PER; ++r) {
         const int idx = tid + r * NT;
-        if (TILE % NT == 0 || idx < TILE) us[(idx / ND) * NDP + padn<N, PAD>(idx % ND)] = v[r];
+        if (TILE % NT == 0 || idx < TILE) us[idx] = v[r];
       }
     } else {
-      for (int idx = tid; idx < ne * NV * ND; idx += NT)
-        us[(idx / ND) * NDP + padn<N, PAD>(idx % ND)] = __ldg(src + idx);
+      for (int idx = tid; idx < ne * NV * ND; idx += NT) us[idx] = __ldg(src + idx);
     }
   }
 };
-
-// issue() and store() back to back.
-template <int N, int NV, int ND, int NDP, int EPB, int NT>
-__device__ __forceinline__ void load_element_tile(const double* src, double* us, int ne,
-                                                  int tid) {
-  ElementTileLoad<N, NV, ND, NDP, EPB, NT> t;
-  t.issue(src, ne, tid);
-  t.store(src, us, ne, tid);
-}
 
 // Element index over the axes != c of the element whose coordinate along
 // `dir` is replaced by `pos` (the neighbour across a face of direction dir).
@@ -551,13 +487,12 @@ __device__ __forceinline__ int eidx_other_shift(const int* I, int c, int dir, in
 // Interface or boundary flux f* at face node `line` of the face (dir, side)
 // of element `el` (surface_flux.hpp:45-271, boundary_set.hpp:70-86), with
 // this element's state at the face node given as `so`.
-template <int DIM, int N, int VF, int SF, bool NS, int NDP>
+template <int DIM, int N, int VF, int SF, bool NS>
 __device__ __forceinline__ void element_face_flux_state(
     const StageArgs<N>& p, const MeshView& M, const FaceState<DIM>& so, const double* us_el,
     int e_own, const int* I, int dir, int side, int line, double gamma, double t_stage, int c0,
     int c1, int c2, double* f) {
   constexpr int NV = DIM + 2, ND = ipow(N, DIM);
-  constexpr bool PAD = NDP != ND;
   const int own_node = line_node<DIM, N>(dir, line, side ? N - 1 : 0);
   const int face = 2 * dir + side;
   const int en = I[6 + face];
@@ -599,7 +534,7 @@ __device__ __forceinline__ void element_face_flux_state(
           double acc = 0.0;
 #pragma unroll
           for (int m = 0; m < N; ++m)
-            acc += us_el[q * NDP + padn<N, PAD>(line_node<DIM, N>(dir, line, m))];
+            acc += us_el[q * ND + line_node<DIM, N>(dir, line, m)];
           ux[q] = acc / (double)N;
         }
       } else {  // slip wall / wall branch of the mixed BC

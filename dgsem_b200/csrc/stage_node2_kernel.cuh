@@ -130,9 +130,9 @@ __device__ __forceinline__ void stage_node2_body(const StageArgs<N>& p) {
   using S = Node2Shape<N, VF>;
   using K = NodeKernelSlots<DIM, VF>;
   constexpr int EPB = NL::EPB, NT = NL::NT, NH = NL::NH;
-  constexpr int NV = S::NV, ND = S::ND, NDP = S::NDP, NF = S::NF, NFACE = S::NFACE,
+  constexpr int NV = S::NV, ND = S::ND, NF = S::NF, NFACE = S::NFACE,
                 NQ = S::NQ, NI = S::NI;
-  static_assert(NDP == ND && !S::XCHG && S::NT == 2 * NT, "shape");
+  static_assert(!S::XCHG && S::NT == 2 * NT, "shape");
   static_assert(S::SM_A == 0 && S::SM_VINV == 0 && S::SM_X == 0, "layout");
   extern __shared__ __align__(128) double smem_node2[];
   double* us = smem_node2;     // [el][var][node]
@@ -162,7 +162,7 @@ __device__ __forceinline__ void stage_node2_body(const StageArgs<N>& p) {
   const bool active = el < ne;
   const bool own_node = M.mij != nullptr && M.info != nullptr;
   const double* tile_src = M.u_in + (int64_t)e0 * NV * ND;
-  ElementTileLoad<N, NV, ND, NDP, EPB, NT> tload;
+  ElementTileLoad<NV, ND, EPB, NT> tload;
   double u2[2][NV];
   double mij_ab[2] = {0.0, 0.0};
   if (own_node) {
@@ -205,20 +205,20 @@ __device__ __forceinline__ void stage_node2_body(const StageArgs<N>& p) {
       const int node = s ? nB : nA;
       if (own_node) {
 #pragma unroll
-        for (int q = 0; q < NV; ++q) us[(el * NV + q) * NDP + node] = u2[s][q];
+        for (int q = 0; q < NV; ++q) us[(el * NV + q) * ND + node] = u2[s][q];
       } else {
 #pragma unroll
-        for (int q = 0; q < NV; ++q) u2[s][q] = us[(el * NV + q) * NDP + node];
+        for (int q = 0; q < NV; ++q) u2[s][q] = us[(el * NV + q) * ND + node];
       }
-      node_prepare<DIM, N, VF, NDP>(M, u2[s], gamma, info + el * NI, node,
-                                    pr + el * NQ * NDP + node, own_node ? &mij_ab[s] : nullptr);
+      node_prepare<DIM, N, VF>(M, u2[s], gamma, info + el * NI, node, pr + el * NQ * ND + node,
+                               own_node ? &mij_ab[s] : nullptr);
     }
   }
   __syncthreads();
 
   // ---- phase 2a: face fluxes ---------------------------------------------
-  node_face_tasks<DIM, N, VF, SF, false, NDP, NT, NQ, NI>(p, M, us, pr, info, sf, e0, ne,
-                                                          tid, gamma, t_stage, c0, c1, c2);
+  node_face_tasks<DIM, N, VF, SF, false, NT, NQ, NI>(p, M, us, pr, info, sf, e0, ne, tid, gamma,
+                                                     t_stage, c0, c1, c2);
 
   // ---- phase 2b: volume term of both nodes -------------------------------
   // every lane runs it (lanes past the last element of a partial tile read
@@ -229,19 +229,15 @@ __device__ __forceinline__ void stage_node2_body(const StageArgs<N>& p) {
   {
     const int ev = active ? el : 0;
     const int* I = info + ev * NI;
-    const double* U = us + ev * NV * NDP;
-    const double* P = pr + ev * NQ * NDP;
+    const double* U = us + ev * NV * ND;
+    const double* P = pr + ev * NQ * ND;
     const double hgm1 = 0.5 * p.inv_gm1;
-    const NodeFluxState<DIM> ownA = load_flux_state<DIM, VF>(U, P, NDP, nA);
-    const NodeFluxState<DIM> ownB = load_flux_state<DIM, VF>(U, P, NDP, nB);
-    node_volume_direction<0, DIM, N, VF, NDP, true, false>(p, M, U, P, I, nA, nA, ownA, hgm1,
-                                                           accA);
-    node_volume_direction<0, DIM, N, VF, NDP, true, false>(p, M, U, P, I, nB, nB, ownB, hgm1,
-                                                           accB);
-    node_volume_direction<1, DIM, N, VF, NDP, true, false>(p, M, U, P, I, nA, nA, ownA, hgm1,
-                                                           accA);
-    node_volume_direction<1, DIM, N, VF, NDP, true, false>(p, M, U, P, I, nB, nB, ownB, hgm1,
-                                                           accB);
+    const NodeFluxState<DIM> ownA = load_flux_state<DIM, VF>(U, P, ND, nA);
+    const NodeFluxState<DIM> ownB = load_flux_state<DIM, VF>(U, P, ND, nB);
+    node_volume_direction<0, DIM, N, VF, true, false>(p, M, U, P, I, nA, ownA, hgm1, accA);
+    node_volume_direction<0, DIM, N, VF, true, false>(p, M, U, P, I, nB, ownB, hgm1, accB);
+    node_volume_direction<1, DIM, N, VF, true, false>(p, M, U, P, I, nA, ownA, hgm1, accA);
+    node_volume_direction<1, DIM, N, VF, true, false>(p, M, U, P, I, nB, ownB, hgm1, accB);
     node2_volume_z<N, VF>(p, M, U, P, I, nA, ownA, ownB, hgm1, accA, accB);
   }
   __syncthreads();
@@ -263,14 +259,14 @@ __device__ __forceinline__ void stage_node2_body(const StageArgs<N>& p) {
       const int node = s ? nB : nA;
       double* acc = s ? accB : accA;
       node_lift<DIM, N>(sf + el * NFACE * NF * NV, node, p.basis.lhat_l0, p.basis.lhat_rN, acc);
-      const double mij = pr[(el * NQ + K::MIJ) * NDP + node];
+      const double mij = pr[(el * NQ + K::MIJ) * ND + node];
       const int64_t gbase = (int64_t)(e0 + el) * NV * ND + node;
       double vals[NV];
 #pragma unroll
       for (int q = 0; q < NV; ++q) {
         const int64_t gi = gbase + (int64_t)q * ND;
         double val = M.c * (acc[q] * mij);
-        if (p.b != 0.0) val = p.b * us[(el * NV + q) * NDP + node] + val;
+        if (p.b != 0.0) val = p.b * us[(el * NV + q) * ND + node] + val;
         if (p.a != 0.0)
           val = p.a * (bulk_n ? stage_n[(el * NV + q) * ND + node] : M.u_n[gi]) + val;
         bad |= !isfinite(val);

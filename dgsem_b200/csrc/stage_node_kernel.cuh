@@ -60,14 +60,12 @@ template <int DIM, int N, int VF, int EPB, bool HG = false, bool NS = false>
 struct NodeShape {
   static constexpr int NV = DIM + 2;
   static constexpr int ND = ipow(N, DIM);
-  static constexpr bool PAD = false;  // unpadded node arrays (see padn)
-  static constexpr int NDP = PAD ? ND + ND / N : ND;
   static constexpr int NF = ipow(N, DIM - 1);
   static constexpr int NFACE = 2 * DIM;
   static constexpr int NQ = NodeKernelSlots<DIM, VF>::NQ;
   static constexpr int NI = 12;
-  static constexpr int SM_U = EPB * NV * NDP;
-  static constexpr int SM_P = EPB * NQ * NDP;
+  static constexpr int SM_U = EPB * NV * ND;
+  static constexpr int SM_P = EPB * NQ * ND;
   // f* [el][face][fn][var]; with shock capturing also the indicator scratch
   static constexpr int SM_F0 = EPB * NFACE * NF * NV;
   static constexpr int SM_F = HG && 2 * EPB * ND > SM_F0 ? 2 * EPB * ND : SM_F0;
@@ -108,17 +106,17 @@ struct NodeFluxState {
 
 template <int DIM, int VF>
 __device__ __forceinline__ NodeFluxState<DIM> load_flux_state(const double* U, const double* P,
-                                                              int NDP, int pn) {
+                                                              int ND, int pn) {
   using K = NodeKernelSlots<DIM, VF>;
   NodeFluxState<DIM> s;
   s.rho = U[pn];
 #pragma unroll
-  for (int d = 0; d < DIM; ++d) s.v[d] = P[(K::V + d) * NDP + pn];
-  s.p = P[K::P * NDP + pn];
+  for (int d = 0; d < DIM; ++d) s.v[d] = P[(K::V + d) * ND + pn];
+  s.p = P[K::P * ND + pn];
   // Chandrashekar loads rho anyway: rho / 2 is exact, so derive it instead
   // of a second shared-memory load (Kennedy-Gruber uses only rho / 2)
-  s.hrho = !K::HALF ? 0.0 : VF == VF_CHANDRASHEKAR ? 0.5 * s.rho : P[K::H_RHO * NDP + pn];
-  s.x = K::HALF ? P[K::X * NDP + pn] : 0.0;
+  s.hrho = !K::HALF ? 0.0 : VF == VF_CHANDRASHEKAR ? 0.5 * s.rho : P[K::H_RHO * ND + pn];
+  s.x = K::HALF ? P[K::X * ND + pn] : 0.0;
   // |v|^2 / 4 = sum (v_d / 2)^2 from the halved velocity, in the summation
   // order of prepare_node: bit for bit the stored value, one load fewer
   s.y = 0.0;
@@ -197,19 +195,18 @@ __device__ __forceinline__ void node_volume_flux(const NodeFluxState<DIM>& L,
 // normal bit for bit).  XB: the whole block executes the call and `xbuf`
 // holds (n-1)/2 * NV * nth doubles; pairs on lines that do not lie in one
 // warp are then shared through it (two block barriers per direction).
-template <int DIR, int DIM, int N, int VF, int NDP, bool WARP_ALL = false, bool XB = false>
+template <int DIR, int DIM, int N, int VF, bool WARP_ALL = false, bool XB = false>
 __device__ __forceinline__ void node_volume_direction(const StageArgs<N>& p, const MeshView& M,
                                                       const double* U, const double* P,
-                                                      const int* I, int node, int pn,
+                                                      const int* I, int node,
                                                       const NodeFluxState<DIM>& own,
                                                       double hgm1, double* acc,
                                                       double* xbuf = nullptr, int tid = 0,
                                                       int nth = 0, bool in_range = true) {
   constexpr int NV = DIM + 2, ND = ipow(N, DIM);
   constexpr bool HALF = NodeKernelSlots<DIM, VF>::HALF;
-  // node-index and shared-memory-index strides along DIR
+  // node-index stride along DIR
   constexpr int SN = DIR == 0 ? 1 : DIR == 1 ? N : N * N;
-  constexpr int SP = NDP == ND ? SN : DIR == 0 ? 1 : DIR == 1 ? N + 1 : N * N + N;
   const int m = DIR == 0 ? node % N : DIR == 1 ? (node / N) % N : node / (N * N);
   const double* jrow[DIM];
   double hja_own[DIM];
@@ -235,7 +232,7 @@ __device__ __forceinline__ void node_volume_direction(const StageArgs<N>& p, con
     if ((SHFL || XCHG) && o > N - o) continue;
     const bool wrap = m + o >= N;
     const int delta = wrap ? o - N : o;  // k - m
-    const NodeFluxState<DIM> other = load_flux_state<DIM, VF>(U, P, NDP, pn + delta * SP);
+    const NodeFluxState<DIM> other = load_flux_state<DIM, VF>(U, P, ND, node + delta * SN);
     double nrm[DIM];
 #pragma unroll
     for (int c = 0; c < DIM; ++c) {
@@ -289,12 +286,12 @@ __device__ __forceinline__ void node_volume_direction(const StageArgs<N>& p, con
 // (volume_flux.hpp:457-509 in 2D, :521-630 in 3D): LLF on the subcell normals
 // at the node's two subcell interfaces, weighted by alpha / w_m (each
 // interface flux is evaluated by both of its nodes).
-template <int DIR, int DIM, int N, int VF, int NDP>
+template <int DIR, int DIM, int N, int VF>
 __device__ __forceinline__ void node_fv_direction(const StageArgs<N>& p, const MeshView& M,
                                                   const double* U, const double* P,
                                                   const int* I, int node, double alpha,
                                                   double* acc) {
-  constexpr int NV = DIM + 2;
+  constexpr int NV = DIM + 2, ND = ipow(N, DIM);
   constexpr int NF = ipow(N, DIM - 1);
   using K = NodeKernelSlots<DIM, VF>;
   const int m = DIR == 0 ? node % N : DIR == 1 ? (node / N) % N : node / (N * N);
@@ -302,15 +299,15 @@ __device__ __forceinline__ void node_fv_direction(const StageArgs<N>& p, const M
                    : DIR == 1 ? node % N + N * (node / (N * N))
                               : node % (N * N);
   auto state = [&](int k) {
-    const int pk = padn<N, (NDP != ipow(N, DIM))>(line_node<DIM, N>(DIR, line, k));
+    const int pk = line_node<DIM, N>(DIR, line, k);
     FaceState<DIM> st;
 #pragma unroll
-    for (int q = 0; q < NV; ++q) st.u[q] = U[q * NDP + pk];
+    for (int q = 0; q < NV; ++q) st.u[q] = U[q * ND + pk];
     const double g = K::HALF ? 2.0 : 1.0;
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) st.v[d] = g * P[(K::V + d) * NDP + pk];
-    st.p = g * P[K::P * NDP + pk];
-    st.a2 = P[K::A * NDP + pk];
+    for (int d = 0; d < DIM; ++d) st.v[d] = g * P[(K::V + d) * ND + pk];
+    st.p = g * P[K::P * ND + pk];
+    st.a2 = P[K::A * ND + pk];
     return st;
   };
   auto normal = [&](int fi, double* nrm) {
@@ -416,30 +413,31 @@ __global__ void element_tables_kernel(const MeshView M, int* info, double* mij) 
 // Per-node data of phase 1 (NodeKernelSlots) from the conserved state u:
 // the (halved) primitive variables, the squared sound speed gamma p / rho and
 // -1/J from the separable metric tables.
-template <int DIM, int N, int VF, int NDP>
+template <int DIM, int N, int VF>
 __device__ __forceinline__ void node_prepare(const MeshView& M, const double* u, double gamma,
                                              const int* I, int node, double* P,
                                              const double* mij_pre = nullptr) {
   using K = NodeKernelSlots<DIM, VF>;
+  constexpr int ND = ipow(N, DIM);
   const NodeState<DIM> s = prepare_node<DIM, VF>(u, gamma);
   const double h = K::HALF ? 0.5 : 1.0;
 #pragma unroll
-  for (int d = 0; d < DIM; ++d) P[(K::V + d) * NDP] = h * s.v[d];
-  P[K::P * NDP] = h * s.p;
+  for (int d = 0; d < DIM; ++d) P[(K::V + d) * ND] = h * s.v[d];
+  P[K::P * ND] = h * s.p;
   // used only by the wave-speed estimate of the surface flux: gamma p (1/rho)
   // is within an ulp of gamma p / rho
-  P[K::A * NDP] = gamma * s.p * s.inv_rho;
+  P[K::A * ND] = gamma * s.p * s.inv_rho;
   if constexpr (K::HALF) {
-    P[K::H_RHO * NDP] = 0.5 * u[0];
-    P[K::X * NDP] = VF == VF_KENNEDY_GRUBER ? 0.5 * s.beta : s.beta;
+    P[K::H_RHO * ND] = 0.5 * u[0];
+    P[K::X * ND] = VF == VF_KENNEDY_GRUBER ? 0.5 * s.beta : s.beta;
   }
-  if constexpr (VF == VF_CHANDRASHEKAR) P[K::Y * NDP] = 0.5 * s.kin;
+  if constexpr (VF == VF_CHANDRASHEKAR) P[K::Y * ND] = 0.5 * s.kin;
   if (mij_pre) {  // element_tables_kernel computed it with the expression below
-    P[K::MIJ * NDP] = *mij_pre;
+    P[K::MIJ * ND] = *mij_pre;
     return;
   }
   const int in = node % N, jn = (node / N) % N, kn = DIM == 3 ? node / (N * N) : 0;
-  P[K::MIJ * NDP] = node_minus_inv_j<DIM, N>(M.tab, I[0], I[1], I[2], in, jn, kn);
+  P[K::MIJ * ND] = node_minus_inv_j<DIM, N>(M.tab, I[0], I[1], I[2], in, jn, kn);
 }
 
 // Surface lifting of one node (surface_integral.hpp:35-154): per direction,
@@ -476,7 +474,7 @@ __device__ __forceinline__ void node_lift(const double* sf_el, int node, double 
 //   2D: one block-stride loop over the tasks in side-major order with the
 //       direction at run time (measured faster there: the boundary branch
 //       of the flux code then exists once).
-template <int DIM, int N, int VF, int SF, bool NS, int NDP, int NT, int NQ, int NI>
+template <int DIM, int N, int VF, int SF, bool NS, int NT, int NQ, int NI>
 __device__ __forceinline__ void node_face_tasks(const StageArgs<N>& p, const MeshView& M,
                                                 const double* us, const double* pr,
                                                 const int* info, double* sf, int e0, int ne,
@@ -487,22 +485,20 @@ __device__ __forceinline__ void node_face_tasks(const StageArgs<N>& p, const Mes
   auto task = [&](int side, int dir, int fe, int fn) {
     const int face = 2 * dir + side;
     const int* I = info + fe * NI;
-    const double* U = us + fe * NV * NDP;
-    const double* P = pr + fe * NQ * NDP;
-    const int opn = padn<N, NDP != ND>(line_node<DIM, N>(dir, fn, side ? N - 1 : 0));
+    const double* U = us + fe * NV * ND;
+    const double* P = pr + fe * NQ * ND;
+    const int opn = line_node<DIM, N>(dir, fn, side ? N - 1 : 0);
     FaceState<DIM> so;
 #pragma unroll
-    for (int q = 0; q < NV; ++q) so.u[q] = U[q * NDP + opn];
+    for (int q = 0; q < NV; ++q) so.u[q] = U[q * ND + opn];
     const double g = K::HALF ? 2.0 : 1.0;
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) so.v[d] = g * P[(K::V + d) * NDP + opn];
-    so.p = g * P[K::P * NDP + opn];
-    so.a2 = P[K::A * NDP + opn];
+    for (int d = 0; d < DIM; ++d) so.v[d] = g * P[(K::V + d) * ND + opn];
+    so.p = g * P[K::P * ND + opn];
+    so.a2 = P[K::A * ND + opn];
     double f[NV];
-    element_face_flux_state<DIM, N, VF, SF, NS, NDP>(p, M, so, U,
-                                                     e0 + fe, I,
-                                                     dir, side, fn, gamma, t_stage, c0, c1, c2,
-                                                     f);
+    element_face_flux_state<DIM, N, VF, SF, NS>(p, M, so, U, e0 + fe, I, dir, side, fn, gamma,
+                                                t_stage, c0, c1, c2, f);
     double* F = sf + ((fe * NFACE + face) * NF + fn) * NV;
 #pragma unroll
     for (int q = 0; q < NV; ++q) F[q] = f[q];
@@ -535,7 +531,7 @@ __device__ __forceinline__ void stage_node_body(const StageArgs<N>& p, int tile 
                 "Navier-Stokes: single mesh; with shock capturing in 2D");
   using S = NodeShape<DIM, N, VF, EPB, HG, NS>;
   using K = NodeKernelSlots<DIM, VF>;
-  constexpr int NV = S::NV, ND = S::ND, NDP = S::NDP, NF = S::NF, NFACE = S::NFACE,
+  constexpr int NV = S::NV, ND = S::ND, NF = S::NF, NFACE = S::NFACE,
                 NQ = S::NQ, NI = S::NI, NT = S::NT;
   extern __shared__ __align__(128) double smem_node[];
   double* us = smem_node;        // [el][var][pnode]
@@ -585,10 +581,9 @@ __device__ __forceinline__ void stage_node_body(const StageArgs<N>& p, int tile 
   // bulk copy that arrives while the block computes (block-uniform decision).
   const int el = tid / ND, node = tid % ND;
   const bool active = el < ne;
-  const int pn = padn<N, S::PAD>(node);
   const bool own_node = M.mij != nullptr && M.info != nullptr;
   const double* tile_src = M.u_in + (int64_t)e0 * NV * ND;
-  ElementTileLoad<N, NV, ND, NDP, EPB, NT> tload;
+  ElementTileLoad<NV, ND, EPB, NT> tload;
   double u[NV];
   double mij_node = 0.0;
   if (own_node) {
@@ -622,13 +617,13 @@ __device__ __forceinline__ void stage_node_body(const StageArgs<N>& p, int tile 
   }
   // node data, squared sound speed and -1/J
   auto node_data = [&](const double* u) {
-    node_prepare<DIM, N, VF, NDP>(M, u, gamma, info + el * NI, node, pr + el * NQ * NDP + pn,
-                                  own_node ? &mij_node : nullptr);
+    node_prepare<DIM, N, VF>(M, u, gamma, info + el * NI, node, pr + el * NQ * ND + node,
+                             own_node ? &mij_node : nullptr);
   };
   if (own_node) {
     if (active) {
 #pragma unroll
-      for (int q = 0; q < NV; ++q) us[(el * NV + q) * NDP + pn] = u[q];
+      for (int q = 0; q < NV; ++q) us[(el * NV + q) * ND + node] = u[q];
       node_data(u);
     }
   } else {
@@ -636,7 +631,7 @@ __device__ __forceinline__ void stage_node_body(const StageArgs<N>& p, int tile 
     __syncthreads();
     if (active) {
 #pragma unroll
-      for (int q = 0; q < NV; ++q) u[q] = us[(el * NV + q) * NDP + pn];
+      for (int q = 0; q < NV; ++q) u[q] = us[(el * NV + q) * ND + node];
       node_data(u);
     }
   }
@@ -653,13 +648,13 @@ __device__ __forceinline__ void stage_node_body(const StageArgs<N>& p, int tile 
     double* bufB = sf + EPB * ND;  // [el][ND]
     const int i0 = node % N, j0 = (node / N) % N, k0 = DIM == 3 ? node / (N * N) : 0;
     if (active) {
-      const double* Ue = us + el * NV * NDP;
+      const double* Ue = us + el * NV * ND;
       if constexpr (DIM == 2)
         bufA[el * ND + node] =
-            hg_node_value(Ue[pn], Ue[NDP + pn], Ue[2 * NDP + pn], Ue[3 * NDP + pn]);
+            hg_node_value(Ue[node], Ue[ND + node], Ue[2 * ND + node], Ue[3 * ND + node]);
       else
-        bufA[el * ND + node] = hg_node_value_3d(Ue[pn], Ue[NDP + pn], Ue[2 * NDP + pn],
-                                                Ue[3 * NDP + pn], Ue[4 * NDP + pn]);
+        bufA[el * ND + node] = hg_node_value_3d(Ue[node], Ue[ND + node], Ue[2 * ND + node],
+                                                Ue[3 * ND + node], Ue[4 * ND + node]);
     }
     __syncthreads();
     if (active) {  // x: sum_ii V(i, ii) ind(.., ii)
@@ -707,8 +702,8 @@ __device__ __forceinline__ void stage_node_body(const StageArgs<N>& p, int tile 
 
   // ---- phase 2a: face fluxes, one task per (element, face, face node) ------
   if (worker)
-    node_face_tasks<DIM, N, VF, SF, NS, NDP, NT, NQ, NI>(p, M, us, pr, info, sf, e0, ne, tid,
-                                                         gamma, t_stage, c0, c1, c2);
+    node_face_tasks<DIM, N, VF, SF, NS, NT, NQ, NI>(p, M, us, pr, info, sf, e0, ne, tid, gamma,
+                                                    t_stage, c0, c1, c2);
 
   // ---- phase 2b: volume term, one thread per node --------------------------
   double acc[NV];
@@ -723,36 +718,33 @@ __device__ __forceinline__ void stage_node_body(const StageArgs<N>& p, int tile 
   if (active || WARP_ALL || S::XCHG) {
     const int ev = active ? el : 0;
     const int* I = info + ev * NI;
-    const double* U = us + ev * NV * NDP;
-    const double* P = pr + ev * NQ * NDP;
-    const NodeFluxState<DIM> own = load_flux_state<DIM, VF>(U, P, NDP, pn);
+    const double* U = us + ev * NV * ND;
+    const double* P = pr + ev * NQ * ND;
+    const NodeFluxState<DIM> own = load_flux_state<DIM, VF>(U, P, ND, node);
     const double hgm1 = 0.5 * p.inv_gm1;
-    node_volume_direction<0, DIM, N, VF, NDP, WARP_ALL, S::XCHG>(p, M, U, P, I, node, pn, own,
-                                                                hgm1, acc, xbuf, tid, NT,
-                                                                worker);
-    node_volume_direction<1, DIM, N, VF, NDP, WARP_ALL, S::XCHG>(p, M, U, P, I, node, pn, own,
-                                                                hgm1, acc, xbuf, tid, NT,
-                                                                worker);
+    node_volume_direction<0, DIM, N, VF, WARP_ALL, S::XCHG>(p, M, U, P, I, node, own, hgm1, acc,
+                                                            xbuf, tid, NT, worker);
+    node_volume_direction<1, DIM, N, VF, WARP_ALL, S::XCHG>(p, M, U, P, I, node, own, hgm1, acc,
+                                                            xbuf, tid, NT, worker);
     if constexpr (DIM == 3)
-      node_volume_direction<2, DIM, N, VF, NDP, WARP_ALL, S::XCHG>(p, M, U, P, I, node, pn, own,
-                                                                  hgm1, acc, xbuf, tid, NT,
-                                                                  worker);
+      node_volume_direction<2, DIM, N, VF, WARP_ALL, S::XCHG>(p, M, U, P, I, node, own, hgm1, acc,
+                                                              xbuf, tid, NT, worker);
   }
   if constexpr (HG) {
     if (active) {
       const int* I = info + el * NI;
-      const double* U = us + el * NV * NDP;
-      const double* P = pr + el * NQ * NDP;
+      const double* U = us + el * NV * ND;
+      const double* P = pr + el * NQ * ND;
       // volume_flux.hpp:817-842: (1 - alpha) DG + alpha FV for troubled elements
       const double alpha = alpha_s[el];
       if (fabs(alpha - 0.0) > p.atol) {
         const double one_m = 1.0 - alpha;
 #pragma unroll
         for (int q = 0; q < NV; ++q) acc[q] *= one_m;
-        node_fv_direction<0, DIM, N, VF, NDP>(p, M, U, P, I, node, alpha, acc);
-        node_fv_direction<1, DIM, N, VF, NDP>(p, M, U, P, I, node, alpha, acc);
+        node_fv_direction<0, DIM, N, VF>(p, M, U, P, I, node, alpha, acc);
+        node_fv_direction<1, DIM, N, VF>(p, M, U, P, I, node, alpha, acc);
         if constexpr (DIM == 3)
-          node_fv_direction<2, DIM, N, VF, NDP>(p, M, U, P, I, node, alpha, acc);
+          node_fv_direction<2, DIM, N, VF>(p, M, U, P, I, node, alpha, acc);
       }
     }
   }
@@ -792,7 +784,7 @@ __device__ __forceinline__ void stage_node_body(const StageArgs<N>& p, int tile 
 
   // ---- phase 3: lifting (surface_integral.hpp:35-154), -1/J, SSPRK3 --------
   node_lift<DIM, N>(sf + el * NFACE * NF * NV, node, p.basis.lhat_l0, p.basis.lhat_rN, acc);
-  const double mij = pr[(el * NQ + K::MIJ) * NDP + pn];
+  const double mij = pr[(el * NQ + K::MIJ) * ND + node];
   const int64_t gbase = (int64_t)(e0 + el) * NV * ND + node;
   bool bad = false;
   double vals[NV];
@@ -801,7 +793,7 @@ __device__ __forceinline__ void stage_node_body(const StageArgs<N>& p, int tile 
     const double du = acc[q] * mij;
     const int64_t gi = gbase + (int64_t)q * ND;
     double val = M.c * du;
-    if (p.b != 0.0) val = p.b * us[(el * NV + q) * NDP + pn] + val;
+    if (p.b != 0.0) val = p.b * us[(el * NV + q) * ND + node] + val;
     if (p.a != 0.0)
       val = p.a * (bulk_n ? stage_n[(el * NV + q) * ND + node] : M.u_n[gi]) + val;
     bad |= !isfinite(val);

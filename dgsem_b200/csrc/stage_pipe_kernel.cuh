@@ -28,7 +28,7 @@ namespace dgsem {
 template <int DIM, int N, int VF, int EPB>
 struct PipeShape {
   using B = NodeShape<DIM, N, VF, EPB>;
-  static constexpr int NV = B::NV, ND = B::ND, NDP = B::NDP, NF = B::NF, NFACE = B::NFACE,
+  static constexpr int NV = B::NV, ND = B::ND, NF = B::NF, NFACE = B::NFACE,
                        NQ = B::NQ, NI = B::NI, NT = B::NT;
   static constexpr int SM_T = EPB * NV * ND;  // one staged tile (unpadded)
   static constexpr size_t smem_bytes =
@@ -47,7 +47,7 @@ template <int DIM, int N, int VF, int SF, int EPB>
 __device__ __forceinline__ void stage_pipe_body(const StageArgs<N>& p, int ntiles) {
   using S = PipeShape<DIM, N, VF, EPB>;
   using K = NodeKernelSlots<DIM, VF>;
-  constexpr int NV = S::NV, ND = S::ND, NDP = S::NDP, NF = S::NF, NFACE = S::NFACE,
+  constexpr int NV = S::NV, ND = S::ND, NF = S::NF, NFACE = S::NFACE,
                 NQ = S::NQ, NI = S::NI, NT = S::NT;
   extern __shared__ __align__(128) double smem_pipe[];
   double* stage_in = smem_pipe;                    // [el][var][node], bulk-copy target
@@ -90,7 +90,6 @@ __device__ __forceinline__ void stage_pipe_body(const StageArgs<N>& p, int ntile
   }
 
   const int el = tid / ND, node = tid % ND;
-  const int pn = padn<N, S::B::PAD>(node);
   uint32_t phase = 0;
   double dacc[3] = {0.0, 0.0, 0.0};  // fused diagnostics of this block's tiles
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x, phase ^= 1u) {
@@ -120,10 +119,10 @@ __device__ __forceinline__ void stage_pipe_body(const StageArgs<N>& p, int ntile
 #pragma unroll
       for (int q = 0; q < NV; ++q) {
         u[q] = stage_in[(el * NV + q) * ND + node];
-        us[(el * NV + q) * NDP + pn] = u[q];
+        us[(el * NV + q) * ND + node] = u[q];
       }
-      node_prepare<DIM, N, VF, NDP>(M, u, gamma, info + el * NI, node, pr + el * NQ * NDP + pn,
-                                    M.mij ? &mij_node : nullptr);
+      node_prepare<DIM, N, VF>(M, u, gamma, info + el * NI, node, pr + el * NQ * ND + node,
+                               M.mij ? &mij_node : nullptr);
     }
     __syncthreads();
     // stage_in is consumed: request the next tile's u_in
@@ -131,8 +130,8 @@ __device__ __forceinline__ void stage_pipe_body(const StageArgs<N>& p, int ntile
       request(&bar_in, stage_in, M.u_in, t + gridDim.x);
 
     // ---- phase 2a: face fluxes ---------------------------------------------
-    node_face_tasks<DIM, N, VF, SF, false, NDP, NT, NQ, NI>(p, M, us, pr, info, sf, e0, ne,
-                                                            tid, gamma, t_stage, c0, c1, c2);
+    node_face_tasks<DIM, N, VF, SF, false, NT, NQ, NI>(p, M, us, pr, info, sf, e0, ne, tid, gamma,
+                                                       t_stage, c0, c1, c2);
 
     // ---- phase 2b: volume term ---------------------------------------------
     double acc[NV];
@@ -145,17 +144,17 @@ __device__ __forceinline__ void stage_pipe_body(const StageArgs<N>& p, int ntile
     if (active || WARP_ALL || XB) {
       const int ev = active ? el : 0;
       const int* I = info + ev * NI;
-      const double* U = us + ev * NV * NDP;
-      const double* P = pr + ev * NQ * NDP;
-      const NodeFluxState<DIM> own = load_flux_state<DIM, VF>(U, P, NDP, pn);
+      const double* U = us + ev * NV * ND;
+      const double* P = pr + ev * NQ * ND;
+      const NodeFluxState<DIM> own = load_flux_state<DIM, VF>(U, P, ND, node);
       const double hgm1 = 0.5 * p.inv_gm1;
-      node_volume_direction<0, DIM, N, VF, NDP, WARP_ALL, XB>(p, M, U, P, I, node, pn, own, hgm1,
-                                                              acc, xbuf, tid, NT);
-      node_volume_direction<1, DIM, N, VF, NDP, WARP_ALL, XB>(p, M, U, P, I, node, pn, own, hgm1,
-                                                              acc, xbuf, tid, NT);
+      node_volume_direction<0, DIM, N, VF, WARP_ALL, XB>(p, M, U, P, I, node, own, hgm1, acc, xbuf,
+                                                         tid, NT);
+      node_volume_direction<1, DIM, N, VF, WARP_ALL, XB>(p, M, U, P, I, node, own, hgm1, acc, xbuf,
+                                                         tid, NT);
       if constexpr (DIM == 3)
-        node_volume_direction<2, DIM, N, VF, NDP, WARP_ALL, XB>(p, M, U, P, I, node, pn, own,
-                                                                hgm1, acc, xbuf, tid, NT);
+        node_volume_direction<2, DIM, N, VF, WARP_ALL, XB>(p, M, U, P, I, node, own, hgm1, acc,
+                                                           xbuf, tid, NT);
     }
     __syncthreads();
 
@@ -166,7 +165,7 @@ __device__ __forceinline__ void stage_pipe_body(const StageArgs<N>& p, int ntile
     }
     if (active) {
       node_lift<DIM, N>(sf + el * NFACE * NF * NV, node, p.basis.lhat_l0, p.basis.lhat_rN, acc);
-      const double mij = pr[(el * NQ + K::MIJ) * NDP + pn];
+      const double mij = pr[(el * NQ + K::MIJ) * ND + node];
       const int64_t gbase = (int64_t)(e0 + el) * NV * ND + node;
       bool bad = false;
       double vals[NV];
@@ -174,7 +173,7 @@ __device__ __forceinline__ void stage_pipe_body(const StageArgs<N>& p, int ntile
       for (int q = 0; q < NV; ++q) {
         const double du = acc[q] * mij;
         double val = M.c * du;
-        if (p.b != 0.0) val = p.b * us[(el * NV + q) * NDP + pn] + val;
+        if (p.b != 0.0) val = p.b * us[(el * NV + q) * ND + node] + val;
         if (with_n) val = p.a * stage_n[(el * NV + q) * ND + node] + val;
         bad |= !isfinite(val);
         M.out[gbase + (int64_t)q * ND] = val;
