@@ -1,9 +1,11 @@
 // Type-erased solver engine: one instantiation per supported template
 // combination (dimension, nodes per direction, volume flux, surface flux,
 // shock capturing, Navier-Stokes).  Each engine carries several launch shapes
-// of the same fused kernel (elements per block, register cap); they compute
-// bitwise-identical results and the autotuner (capi.cu: dgsem_autotune)
-// picks the fastest for a mesh.  The C ABI context owns one engine.
+// of the same right-hand side; shapes 0-2 give the same bits, the others agree
+// with them to rounding (other orders of summation, and logarithms where 0-2
+// take a series).  So the autotuner's choice (capi.cu: dgsem_autotune), which is
+// by time, can change the last bits of a result; a fixed shape never does.
+// The C ABI context owns one engine.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -41,7 +43,9 @@ struct EngineConfig {
   double* visc;             // Navier-Stokes contravariant viscous flux (br1_kernel.cuh)
   double* grad;             // adjoint: velocity gradient written with it (may be null)
   // per-element info (node_element_info layout, 12 ints per element) and
-  // -1/J per node [E][n^d], computed once per context (may be null)
+  // -1/J per node [E][n^d], computed once per context.  The line shapes and the
+  // viscous flux kernel read them unconditionally; null only in the shared
+  // configuration of a batch group, whose launches take them from the mesh views
   const int* elem_info;
   const double* mij;
   // failure-path testing (StageArgs::wait_limit_ns / skip_tile_copy)
@@ -69,7 +73,7 @@ class EngineBase {
                             double* alpha_out, cudaStream_t s, double* diag = nullptr) = 0;
   // number of diag slots (blocks) the last stage launch with diag wrote
   virtual int64_t last_diag_slots() const = 0;
-  // Fills the per-mesh tables of the node-parallel kernels (EngineConfig::
+  // Fills the per-mesh tables of the stage kernels (EngineConfig::
   // elem_info / MeshView::info, 12 ints per element; ::mij, -1/J per node)
   // of the mesh `m` (its cells, periodicity, element count and metric
   // tables) on stream s.
@@ -193,10 +197,14 @@ struct NodeLaunch {
 
 // Launches a stage kernel with programmatic stream serialization: the GPU
 // may schedule its blocks while the previous kernel on `s` drains (hiding the
-// launch gap between the three stages of a step); the kernel's first
-// instruction, griddepcontrol.wait (stage_dependency_sync), holds every block
-// until that kernel has completed and flushed its writes.  After a copy, a
-// memset or an event the launch is ordered as usual.
+// launch gap between the three stages of a step); griddepcontrol.wait
+// (stage_dependency_sync) holds every block until that kernel has completed and
+// flushed its writes.  After a copy, a memset or an event the launch is ordered
+// as usual.  Before the wait a kernel reads only what no kernel of a step
+// writes: its arguments, the metric tables, element info and -1/J
+// (element_tables_kernel writes the last two at creation, which ends with a
+// device synchronisation), mesh views and tile lists (host copies).  Whoever
+// writes one of these on the device has to synchronise before the next launch.
 template <class... P, class... A>
 void launch_stage_kernel(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
                          cudaStream_t s, A&&... args) {
@@ -305,8 +313,8 @@ class Engine final : public EngineBase {
 
   // Shape 0 runs the split form on meshes that give the sweep fewer than
   // split_waves() waves: `nelem` / EPW warps on WPB * MINB warp slots per SM.
-  // A sweep's time is one lane's chain per wave; the split form's chain is a
-  // third of it, but its blocks fill the GPU sooner.  Both give the same bits.
+  // A sweep's time is one lane's chain per wave; the split form's chain is about
+  // half of it, but its blocks fill the GPU sooner.  Both give the same bits.
   // Measured on a B200 (1776 slots, 1184 at long lines) at 14 sizes of 0.1 to 3.3
   // waves per form; split / sweep time at the two sizes around the crossing, the
   // last column the crossing in waves:

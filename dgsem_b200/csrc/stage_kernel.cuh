@@ -78,8 +78,9 @@ struct MeshView {
   int nelem;
   int periodic[3];
   DeviceTables tab;
-  // optional per-mesh tables of the node-parallel kernels (null: computed in
-  // the kernel): element info, 12 ints per element, and -1/J per node
+  // element info, 12 ints per element, and -1/J per node.  The line shapes
+  // need them (tables 32-byte aligned: they are read as vectors); the
+  // node-parallel kernels compute them where they are null
   const int* info;
   const double* mij;
 };
@@ -432,10 +433,11 @@ __device__ double hg_alpha_2d(const double* us_el, int ND, const BasisConst<N>& 
 // ---------------------------------------------------------------------------
 // Programmatic dependent launch: the stage kernels are launched with
 // programmatic stream serialization, so a stage kernel may be scheduled while
-// the previous kernel on its stream is still draining.  Each block first
-// waits for that kernel's completion and memory flush (before it reads any
-// kernel argument array), then lets the next kernel be scheduled.  Both
-// instructions are no-ops in a normal launch.
+// the previous kernel on its stream is still draining.  Each block waits for
+// that kernel's completion and memory flush before it reads or writes anything
+// a kernel of a step writes (launch_stage_kernel lists what may be read
+// earlier), then lets the next kernel be scheduled.  Both instructions are
+// no-ops in a normal launch.
 __device__ __forceinline__ void stage_dependency_sync() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -20,31 +20,34 @@
 // each end face belongs to the line that holds its own state, and the pairs
 // of a line are independent instruction streams that cover the FP64 latency.
 // That halves the instructions per node; what then bounds the kernel is the
-// latency of its global loads and of instruction fetch, so
+// latency of its global loads, so
 //   * the loads a direction needs (neighbour traces, metric terms, normals)
 //     are issued together before its volume term, u_n is brought into L2 at
 //     kernel start, and the state is read once (everything later comes from
 //     shared memory);
 //   * the volume term is one straight block without branches: reciprocals and
-//     roots are branch-free (physics.cuh: recip, root) and the logarithmic
+//     roots are branch-free (physics.cuh: recip_ulp, root) and the logarithmic
 //     means take their series for every pair; a line with a pair outside the
 //     series' range repeats its volume term (LineMean).
 //
 // Shared memory of a warp, planes of doubles [slot][element][node]: the NV
 // conserved variables, 1 / (2 rho), p, Chandrashekar: rho / p; then the NV
-// planes of R.  Node positions are swizzled for n = 4 (line_slot), otherwise
+// planes of R.  Node positions are swizzled for n = 4 (LinePos), otherwise
 // x lines have an odd stride, so that the lines of every direction fall on
 // distinct banks.
 //
 // Measured against the former line-per-direction kernel (one thread per line,
 // one direction per thread, block barriers, 7.5 M warp instructions per TGV
-// 16^3 stage, here 4.5 M) and against one thread per node, B200, us per stage:
+// 16^3 stage, here 4.4 M) and against one thread per node, B200, us per stage
+// (the sweep when it was first measured; with the rounded reciprocals 0.5-2 %
+// more):
 //   KH 1024^2 Ranocha        1181 -> 432   (thread per node 708)
 //   TGV 16^3 Kennedy-Gruber  23.3 -> 13.4  (17.9)
 //   TGV 32^3 Chandrashekar    365 -> 97    (181)
-//   vortex n = 6, 97 x 61    45.9 -> 27.2  (17.0: too few warps in flight)
 //   3D shock capturing n = 5, 1287 elements  29.3 -> 19.0
-// TGV 32^3 then runs the FP64 pipe 51 % of the time at 9.4 TB/s out of L2.
+// ncu on TGV 32^3 Chandrashekar: FP64 pipe 50-52 % of the time, 6.7-8.9 TB/s out
+// of L2, 0.42-0.43 instructions per cycle and scheduler; the longest stall is the
+// global load (1.6-2.0 of 6.5-6.8 cycles between a warp's instructions).
 //
 // Scaling by powers of two is exact, so averages are formed from halved
 // velocities and the pair normal Ja_i + Ja_k, and the factors are collected
@@ -1177,7 +1180,7 @@ __global__ void __launch_bounds__(32 * WPB, MINB) stage_line_kernel(const __grid
 //          alpha; then warp d: blend, lifting, viscous terms -> its planes R_d;
 //   store  the group's nodes, one per thread: R_0 + R_1 [+ R_2], -1/J, SSPRK3
 //          combination.
-// The chain of dependent instructions of a lane is a third of the line
+// The chain of dependent instructions of a lane is about half of the line
 // sweep's; every sum is formed in the same order, so the results are the line
 // sweep's bit for bit.
 // ---------------------------------------------------------------------------

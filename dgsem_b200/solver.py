@@ -361,8 +361,9 @@ class StructuredSolver:
         C.check(C.lib().dgsem_check_finite(self._ctx), "dgsem_check_finite")
 
     def autotune(self, u: torch.Tensor, retime: bool = False):
-        """Picks the fastest launch shape for this mesh (results are identical
-        across shapes); returns (variant, per-variant ms or None)."""
+        """Picks the fastest launch shape for this mesh (results agree across
+        shapes to rounding, bit for bit within 0-2); returns (variant,
+        per-variant ms or None)."""
         chosen = ctypes.c_int()
         times = (ctypes.c_double * 7)() if retime else None
         C.check(C.lib().dgsem_autotune(self._ctx, _ptr(u), ctypes.byref(chosen), times),
