@@ -316,28 +316,27 @@ class Engine final : public EngineBase {
   // A sweep's time is one lane's chain per wave; the split form's chain is about
   // half of it, but its blocks fill the GPU sooner.  Both give the same bits.
   // Measured on a B200 (1776 slots, 1184 at long lines) at 14 sizes of 0.1 to 3.3
-  // waves per form; split / sweep time at the two sizes around the crossing, the
-  // last column the crossing in waves:
-  //   2D Chandrashekar, vortex  n = 4: 0.94 at 0.95, 1.07 at 1.20    1.05
-  //                             n = 2, 3, 5-8: between 0.93 and 1.05
-  //      KH, HLLC or Ranocha, n = 4: 0.91, 0.88 at 0.70, 1.01 at 0.85  0.84
-  //      Kennedy-Gruber n = 4   0.95 at 0.50, 1.15 at 0.70           0.55
-  //      viscous n = 4, 5, 8    1.01, 0.98, 1.02 at 0.70             0.7
-  //   2D shock capturing, KH    n = 2, 3, 4: 1.02, 1.10, 1.21 at 0.85  0.65-0.8
-  //      double Mach n = 4      0.81 at 0.85, 0.98 at 2.1, 1.05 at 2.6  2.2
-  //                             n = 5: 0.92 at 0.50, 1.10 at 0.70    0.6
-  //                             n = 6, 7, 8: 0.92 at 0.20, 1.08 at 0.35  0.28
-  //      viscous n = 3, 4, 5    0.72 at 0.20, 1.12 at 0.35, 1.10 at 0.7  0.2-0.35
-  //   3D n = 2, 3, 4            0.67, 0.89, 0.74 at 0.20, 0.94, 1.13, 0.94 at
-  //                             0.35, 0.98, 1.04, 1.08 at 0.50       0.3-0.5
-  //      n = 5                  0.97 at 0.68, 1.12 at 0.84 (0.91 at 1.02, where
-  //                             the sweep starts its second wave)    0.7
-  //      shock capturing n = 2-4: 0.84 at 0.20, 1.10 at 0.35         0.28
-  //                             n = 5: 0.93 at 0.49, 1.14 at 0.68    0.55
-  //      viscous n = 2-4        0.81-1.04 at 0.20, 0.96-1.13 at 0.35  0.2-0.4
-  // Steep lines lengthen the sweep's chain, so shock capturing at n <= 4 crosses
-  // anywhere from 0.65 (smooth) to 2.2 waves (Mach 10): 0.85 loses at most a
-  // quarter at either.
+  // waves per form; split / sweep time on both sides of the line, at waves:
+  //   2D Chandrashekar, vortex    n = 4: 0.94 at 0.95, 1.07 at 1.20
+  //                               n = 2, 3, 5-8: 0.94-1.04 at 0.95, 1.01-1.16 at 1.2
+  //      Ranocha, HLLC (KH), n = 4  0.88, 0.91 at 0.70, 1.03, 1.10 at 0.95
+  //      Kennedy-Gruber           n = 2, 3: 0.87, 0.83 at 0.70, 1.00 at 0.85
+  //                               n = 4, 5, 6: 0.95, 0.79, 0.94 at 0.50, 1.15, 0.95,
+  //                               0.98 at 0.70, 1.27, 1.16, 1.17 at 0.85
+  //                               n = 7, 8: 0.75, 0.68 at 0.20, 1.16, 1.06 at 0.50
+  //      viscous                  n = 3: 0.92 at 0.70, 1.00 at 0.85
+  //                               n = 4, 5, 8: 1.01, 0.98, 1.02 at 0.70
+  //   3D n = 2, 4                 0.94, 0.94 at 0.35, 0.98, 1.08 at 0.50
+  //      n = 3                    0.89 at 0.20, 1.13 at 0.35 (Kennedy-Gruber 0.90 at 0.50)
+  //      n = 5                    0.97 at 0.68, 1.12 at 0.84 (0.91 at 1.02, where the
+  //                               sweep starts its second wave); viscous 0.96, 1.05
+  // With shock capturing the line depends on the flow, because steep lines
+  // lengthen the sweep's chain: the two crossings are, in waves,
+  //   2D, Kelvin-Helmholtz / double Mach   n = 2, 3, 4: 0.8, 0.8, 0.7 / 1.0, 1.6, 2.0
+  //                               n = 5: 0.6 / 1.7;  n = 6, 8: 0.3, 0.3 / 1.7, 2.2
+  //   2D viscous KH               n = 3, 4, 5, 8: 0.3, 0.2, 0.3, 0.5
+  //   3D Taylor-Green             n = 2, 3, 4, 5: 0.27, 0.27, 0.3, 0.55
+  // and the line lies where neither loses more than 1.45 (2D) or 1.2 (3D).
   void set_mesh_size(int64_t nelem) override {
     using L = LineLaunch<DIM, N, 0>;
     int dev = 0, sms = 0;
@@ -349,10 +348,11 @@ class Engine final : public EngineBase {
     load_variant(variant_);
   }
   static constexpr double split_waves() {
-    if (DIM == 3) return N == 5 ? (HG ? 0.55 : 0.7) : 0.3;
-    if (NS) return HG ? 0.3 : 0.7;
-    if (HG) return N <= 4 ? 0.85 : N == 5 ? 0.6 : 0.28;
-    return VF == VF_KENNEDY_GRUBER ? 0.55 : 0.95;
+    if (DIM == 3) return N <= 4 ? 0.4 : HG ? 0.6 : 0.7;
+    if (HG) return N <= 4 ? 1.13 : N > 5 ? 0.68 : NS ? 0.45 : 0.6;
+    if (NS) return N <= 3 ? 0.8 : 0.7;
+    if (VF == VF_KENNEDY_GRUBER) return N <= 3 ? 0.85 : N <= 6 ? 0.68 : 0.4;
+    return N <= 5 ? 1.0 : 0.95;
   }
 
   // node-parallel shapes: split form with shock capturing or with the
