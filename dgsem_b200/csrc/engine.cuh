@@ -275,10 +275,14 @@ class Engine final : public EngineBase {
 
   // Loads and configures the kernels of one launch shape (and of its batched
   // and fallback forms), once per engine: only shapes that are selected, since
-  // a kernel's code goes to the device at its first use.
+  // a kernel's code goes to the device at its first use.  On the device the
+  // engine was created for, whichever is current in the call that selects.
   void load_variant(int v) {
     if (loaded_ & (1u << v)) return;
     loaded_ |= 1u << v;
+    int current = device_;
+    cudaGetDevice(&current);
+    if (current != device_) cudaSetDevice(device_);
     auto attr = [](auto kernel, size_t smem) {
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     };
@@ -309,6 +313,7 @@ class Engine final : public EngineBase {
       if (v == 5) attr(pipe_kernel(), PSh::smem_bytes);
     if constexpr (kNode2)
       if (v == 6) attr(node2_kernel(), Node2Shape<N, VF>::smem_bytes);
+    if (current != device_) cudaSetDevice(current);
   }
 
   // Shape 0 runs the split form on meshes that give the sweep fewer than
@@ -339,9 +344,9 @@ class Engine final : public EngineBase {
   // and the line lies where neither loses more than 1.45 (2D) or 1.2 (3D).
   void set_mesh_size(int64_t nelem) override {
     using L = LineLaunch<DIM, N, 0>;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int sms = 0;
+    cudaGetDevice(&device_);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_);
     const int64_t warps = (nelem + LG::EPW - 1) / LG::EPW;
     split_ = (double)warps < split_waves() * (sms * L::WPB * L::MINB);
     loaded_ &= ~1u;
@@ -559,6 +564,7 @@ class Engine final : public EngineBase {
   int variant_ = 0;
   bool split_ = false;   // shape 0 runs the split form (set_mesh_size)
   unsigned loaded_ = 0;  // launch shapes configured so far (load_variant)
+  int device_ = 0;       // device of the creation (set_mesh_size)
   mutable int64_t pipe_blocks_ = 0;
   mutable int64_t last_grid_ = 0;  // blocks of the last single-mesh stage launch
   int64_t last_diag_slots_ = 0;

@@ -61,6 +61,8 @@ CASES = [
     _case(2, 2, (8, 6), SPLIT, viscous=True, bc="walls", walls=CHANNEL),
     _case(2, 4, (8, 6), SPLIT, viscous=True, bc="walls", walls=BOX),
     _case(2, 5, (8, 6), SPLIT, viscous=True, bc="walls", walls=CHANNEL),
+    _case(2, 4, (1, 7), SPLIT, viscous=True, bc="walls", walls=BOX),
+    _case(2, 3, (7, 1), SPLIT, hg=True, viscous=True, bc="walls", walls=BOX),
     _case(2, 4, (149, 133), SWEEP, viscous=True, bc="walls", walls=CHANNEL),
     _case(2, 5, (127, 121), SWEEP, viscous=True, bc="walls", walls=BOX),
     _case(2, 4, (137, 131), SWEEP, hg=True, viscous=True, bc="walls", walls=CHANNEL),
