@@ -34,13 +34,15 @@ struct NodeState {
 // Branch-free reciprocals, quotient and square root of normal numbers from the
 // hardware's approximations (rcp.approx.ftz.f64, rsqrt.approx.ftz.f64, about
 // 20 bits):
-//   recip_ulp  r (1 + e + e^2) with e = 1 - a r (third-order Newton-Schulz step):
-//              the rounded reciprocal or, in 3e-4 of the cases, its neighbour
+//   recip_ulp  r (1 + e + e^2) with e = 1 - a r (third-order step of G. Schulz's
+//              iteration, ZAMM 13, 1933): the rounded reciprocal or, in 3e-4 of
+//              the cases, its neighbour
 //   recip      r1 + r1 (1 - a r1) with r1 = recip_ulp(a): the rounded reciprocal
 //              (P. Markstein, IBM J. Res. Dev. 34, 1990: every a whose
 //              significand is not all ones)
 //   quotient   q = a (1/b), then q + (a - q b) (1/b) (the same paper)
-//   root       one Goldschmidt step, then g + h (x - g^2)
+//   root       one step of R. E. Goldschmidt's iteration (MIT thesis, 1964) for
+//              g = sqrt(x) and h = 1 / (2 g), then g + h (x - g^2)
 // tests/test_gpu_scalar_math.py compares them with the rounded results over
 // random significands and exponents.  Arguments must be normal with normal
 // reciprocals: zero, infinite and subnormal ones give a NaN, except that root
